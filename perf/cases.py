@@ -17,6 +17,7 @@ are those of the model configurations (smaller vocabularies where the head has a
 from __future__ import annotations
 
 import torch
+import torch.utils.checkpoint
 
 from infinitrain_b200.autocast import AutocastGuard
 from infinitrain_b200.datatype import DataType
@@ -264,3 +265,115 @@ def tolerance(case):
     if case["kind"] == "attention":
         return {"rel": 1.4e-2, "max": 0.9}
     return {"rel": 1.2e-2, "max": 4e-2}
+
+
+# --------------------------------------------------------------------------- the same in 64 bits
+def _rotate64(x, theta):
+    """RoPE on interleaved pairs: x [B, T, heads, D]."""
+    T, D = x.shape[1], x.shape[3]
+    inv = theta ** (-torch.arange(0, D, 2, dtype=torch.float64, device=x.device) / D)
+    angle = torch.outer(torch.arange(T, dtype=torch.float64, device=x.device), inv)[None, :, None]
+    a, b = x[..., 0::2], x[..., 1::2]
+    return torch.stack((a * angle.cos() - b * angle.sin(), a * angle.sin() + b * angle.cos()), dim=-1).flatten(-2)
+
+
+def _attend64(q, k, v):
+    """Causal attention of [T, heads, D] queries on [T, D] keys and values."""
+    T, D = k.shape
+    future = torch.ones((T, T), dtype=torch.bool, device=k.device).triu(1)
+    s = torch.einsum("thd,sd->hts", q, k) * D ** -0.5
+    return torch.einsum("hts,sd->thd", s.masked_fill(future, float("-inf")).softmax(-1), v)
+
+
+def _attention64(qkv, heads, kv_heads, theta):
+    """Self-attention on a packed projection, one key-value head of one sequence at a time (its scores are computed
+    again for the backward pass)."""
+    B, T, width = qkv.shape
+    D = width // (heads + 2 * kv_heads)
+    q, k, v = qkv.view(B, T, -1, D).split((heads, kv_heads, kv_heads), dim=2)
+    if theta:
+        q, k = _rotate64(q, theta), _rotate64(k, theta)
+    group = heads // kv_heads
+    again = torch.utils.checkpoint.checkpoint
+    rows = [torch.cat([again(_attend64, q[b, :, h * group:(h + 1) * group], k[b, :, h], v[b, :, h], use_reentrant=False)
+                       for h in range(kv_heads)], dim=1) for b in range(B)]
+    return torch.stack(rows).flatten(2)
+
+
+def _norm64(x, weight, bias, eps):
+    if bias is None:
+        return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * weight
+    return torch.nn.functional.layer_norm(x, x.shape[-1:], weight, bias, eps)
+
+
+def _logits64(cfg, weights, ids, lora_scale):
+    """Logits of a GPT-2 or LLaMA-3 model; ``weights`` maps the state dict's names to 64-bit tensors."""
+    F = torch.nn.functional
+
+    def linear(x, name):
+        y = F.linear(x, weights[name + ".weight"], weights.get(name + ".bias"))
+        if name + ".lora_A" in weights:
+            y = y + lora_scale * F.linear(F.linear(x, weights[name + ".lora_A"]), weights[name + ".lora_B"])
+        return y
+
+    def norm(x, name):
+        return _norm64(x, weights[name + ".weight"], weights.get(name + ".bias"), cfg.norm_eps)
+
+    gpt = "transformer.wpe.weight" in weights
+    x = F.embedding(ids, weights["transformer.wte.weight"])
+    if gpt:
+        x = x + weights["transformer.wpe.weight"][:ids.shape[1]]
+    for i in range(cfg.n_layer):
+        h = f"transformer.h.{i}."
+        qkv = linear(norm(x, h + "ln_1"), h + "attn.c_attn")
+        x = x + linear(_attention64(qkv, cfg.n_head, cfg.n_kv_head, 0 if gpt else cfg.rope_theta), h + "attn.c_proj")
+        y = norm(x, h + "ln_2")
+        if gpt:
+            y = F.gelu(linear(y, h + "mlp.c_fc"), approximate="tanh")
+        else:
+            y = linear(y, h + "mlp.c_fc") * F.silu(linear(y, h + "mlp.c_fc2"))
+        x = x + linear(y, h + "mlp.c_proj")
+    return linear(norm(x, "transformer.ln_f"), "lm_head")
+
+
+def _model64(case, seed):
+    if case.get("graph"):
+        return None         # its state has taken warm-up steps already
+    state = prepare(case, seed)
+    named = state["model"].StateDict()
+    leaves = {}             # by address: tied weights are one leaf
+    for p in state["model"].parameters():
+        leaves[p.data_ptr()] = p.detach().double().requires_grad_(case["kind"] == "train" and p.requires_grad)
+    weights = {name: leaves[t.data_ptr()] for name, t in named.items() if t.data_ptr() in leaves}
+    logits = _logits64(_config(case), weights, state["x"], 2.0)
+    if case["kind"] == "eval":
+        return logits
+    loss = torch.nn.functional.cross_entropy(logits.flatten(0, 1), state["y"].flatten())
+    del logits
+    loss.backward()
+    flat = next(p for p in state["model"].parameters() if p.requires_grad)._itb_flat_buffer
+    updated, gradients = (torch.zeros(flat.param_buffer.shape, dtype=torch.float64, device=loss.device) for _ in range(2))
+    for p, (begin, end, _) in zip(flat.params, flat.layout.param_ranges):
+        w = leaves[p.data_ptr()]
+        g = w.grad
+        gradients[begin:end] = g.flatten()
+        # the first AdamW step: both corrected moments are the gradient's own
+        w = w.detach()
+        updated[begin:end] = (w - 1e-4 * (g / (g.abs() + 1e-8) + 0.1 * w)).flatten()
+    return {"loss": loss.detach(), "weights": updated, "gradients": gradients}
+
+
+def exact(case, seed):
+    """What ``run`` returns, by plain torch operations in 64 bits."""
+    if case["kind"] in ("train", "eval"):
+        return _model64(case, seed)
+    state = prepare(case, seed)
+    if case["kind"] == "attention":
+        qkv = state["qkv"].detach().double().requires_grad_()
+        out = _attention64(qkv, case["heads"], case["kv_heads"], 500000.0 if case["rope"] else 0)
+        (dqkv,) = torch.autograd.grad(out, qkv, state["dout"].double())
+        return out.detach(), dqkv
+    x, weight = (state[k].detach().double().requires_grad_() for k in ("x", "weight"))
+    loss = torch.nn.functional.cross_entropy((x @ weight.T)[0], state["target"][0])
+    dx, dw = torch.autograd.grad(loss, (x, weight))
+    return loss.detach(), dx, dw
