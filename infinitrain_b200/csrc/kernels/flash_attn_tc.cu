@@ -6,18 +6,29 @@
 //
 //   S^T[n,m]  = K[n,:] . Q[m,:]            tcgen05.mma  K (K-major)  x Q (K-major)   -> TMEM cols 0..127
 //   dP^T[n,m] = V[n,:] . dO[m,:]           tcgen05.mma  V            x dO            -> TMEM cols 128..255
-//   P^T = exp2(S^T c - lse[m]),  dS^T = P^T (dP^T - delta[m])      256 threads, half a key row each;
-//                                          written as bf16 to shared memory in the swizzled operand layout
-//   dV[n,d] += P^T[n,m]  dO[m,d]           tcgen05.mma  P^T (K-major)  x dO (MN-major) -> TMEM cols 256..
+//   P^T  = exp2(S^T c - lse[m])            8 warps, half a key row per thread; bf16 over the spent S^T in TMEM
+//   dV[n,d] += P^T[n,m]  dO[m,d]           tcgen05.mma  P^T (from TMEM) x dO (MN-major) -> TMEM cols 256..
+//   dS^T = P^T (dP^T - delta[m])           the same warps; bf16 to shared memory in the swizzled operand layout
+//   dQ[m,d]  = dS[m,n]   K[n,d]            tcgen05.mma  dS^T read MN-major x K (MN-major) -> TMEM; four warps of
+//                                          their own read it out and add it to the fp32 dQ buffer by TMA
 //   dK[n,d] += dS^T[n,m] Q[m,d]            tcgen05.mma  dS^T (K-major) x Q  (MN-major) -> TMEM cols 256+D..
-//   dQ[m,d]  = dS[m,n]   K[n,d]            tcgen05.mma  dS^T read MN-major x K (MN-major) -> TMEM, then added
-//                                          to the fp32 dQ buffer with vector reductions
 //
-// Warp roles: warp 0 issues the TMA loads, warp 1 the MMAs, warps 2-9 do the softmax recomputation
-// and the TMEM read-outs (two warps per TMEM lane quarter, each taking half of the columns).  With
-// head size 64 dQ has TMEM columns of its own, so S^T / dP^T of the next tile are computed while the
-// softmax warps still read dQ out; with head size 128 dQ overwrites the spent S^T.  Every wait is
-// bounded; a wait that gives up records a code in the status word and the CTA drains without
+// The softmax warps, the tensor core and the dQ read-out each work on a different part of the chain: the MMA
+// thread issues dV(i) and S(i+1) when P(i) is there, dP(i+1), dQ(i) and dK(i) when dS(i) is there, so S(i+1) is
+// computed under the dS phase of tile i, dP(i+1) under the P phase of tile i+1, and dQ(i) is read out meanwhile.
+// MMAs complete in the order of issue, so s_full(i+1) says that dV(i) has read P(i).  With head size 64 dQ has
+// TMEM columns of its own; with head size 128 it takes the spent dP's, so dP(i+1) comes after dQ(i) and waits for
+// its read-out.
+//
+// What bounds it: the exponentials (16 per cycle and SM: 1024 cycles a tile) and the five contractions (1280
+// cycles a tile at head size 64, 2560 at 128).
+// Measured (this kernel alone, causal): 16 x 1024 tokens, 12 heads of 64: 280 us when one warp set walked the whole
+// chain of a tile, one CTA per key tile; 147 us now.  1 x 8192, 32 query and 8 KV heads of 128: 3018 -> 1400 us.
+// 1 x 2048, 32 / 8 heads of 64: 292 -> 75 us.  A tile takes 3260 cycles at head size 64 and 5000 at 128, where shared
+// memory is busy most of the time: 288 KB of operands, 128 KB for dQ's way out and 96 KB of loads and dS a tile at
+// 128 bytes a cycle are 4100 cycles.
+//
+// Every wait is bounded; a wait that gives up records a code in the status word and the CTA drains without
 // touching the tensor pipe again.
 //
 // The reference composes attention from batched cuBLAS matmuls, a mask and a 3-pass softmax and
@@ -42,8 +53,7 @@ int make_tmap_f32_3d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t
 
 namespace fatc {
 
-constexpr int kThreads = 320;     // TMA warp, MMA warp, 8 softmax / read-out warps
-constexpr int kSoftmaxThreads = 256;
+constexpr int kThreads = 512;     // 8 softmax warps, 4 dQ read-out warps, TMA warp, MMA warp, two idle warps
 constexpr int kAtom = 128 * 128;   // bytes of one [128 rows][64 x bf16] swizzled block
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -52,7 +62,7 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ void softmax_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void readout_warps_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 __device__ __forceinline__ uint4 pack8(const float* v) {
   uint4 u;
@@ -62,78 +72,148 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return u;
 }
 
+// A wait of a whole warp: bounded, and all its lanes get the same answer.  The abort flag is looked at only while
+// there is something to wait for: a wait that finds its phase complete sits in the chain of every tile.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  for (uint32_t i = 0; i < kMbarPollLimit; ++i) {
+    if (__all_sync(~0u, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(~0u, *abort_flag != 0)) return false;
+    if (i > 64) __nanosleep(32);
+  }
+  return false;
+}
+
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
 template <int D>
 struct BwdCfg {
   static constexpr int kAtoms = D / 64;
   static constexpr int kTile = kAtoms * kAtom;          // one [128][D] bf16 tile
-  static constexpr int kQStages = D == 64 ? 2 : 1;
+  static constexpr int kdOStages = D == 64 ? 2 : 1;     // dO(i) is spent at dV(i), early enough for one stage
+  static constexpr int kKvStages = D == 64 ? 2 : 1;     // head size 64 has room to load the next item's K and V early
   static constexpr int kOffK = 0;
-  static constexpr int kOffV = kTile;
-  static constexpr int kOffQ = 2 * kTile;
-  static constexpr int kOffdO = kOffQ + kQStages * kTile;
-  static constexpr int kOffP = kOffdO + kQStages * kTile;    // [2 m-chunks][128 n][64 m]
-  static constexpr int kOffdS = kOffP + 2 * kAtom;
-  static constexpr int kOffStat = kOffdS + 2 * kAtom;        // lse*log2e [2][128], delta [2][128]
+  static constexpr int kOffV = kTile;                        // stage s of K and V: 2 * kTile * s further
+  static constexpr int kOffQ = 2 * kKvStages * kTile;        // two stages: S(i+1) is issued before dK(i)
+  static constexpr int kOffdO = kOffQ + 2 * kTile;
+  static constexpr int kOffdS = kOffdO + kdOStages * kTile;  // [2 m-chunks][128 n][64 m]
+  static constexpr int kOffStage = kOffdS + 2 * kAtom;       // dQ on its way out: two fp32 [128][32] blocks
+  static constexpr int kOffStat = kOffStage + 2 * kAtom;     // lse*log2e [2][128], delta [2][128]
   static constexpr int kOffBar = kOffStat + 4 * 128 * 4;
-  static constexpr int kSmem = kOffBar + 12 * 8 + 16;
+  static constexpr int kSmem = kOffBar + 22 * 8 + 16;
+  static_assert(kSmem <= 232448, "shared memory of one SM");
 };
 
+// What the roles of a CTA walk over: items of (128 keys, KV head, share of its query tiles, batch), each with the
+// (query head of the group, query tile) pairs that meet its keys.
+//
+// The pairs of one key tile and KV head are dealt out to `nparts` items in turn (a.bwd_parts > 1 when whole ones
+// would leave SMs idle: few key tiles, one KV head per rank under tensor parallelism); each then adds its dK / dV
+// into fp32 accumulators instead of writing them.  With a causal mask the items of the first keys have the most
+// tiles: items are ordered by that and dealt out to the CTAs to and fro, so that each gets about the same.
+struct BwdItems {
+  int nparts, width, total, n_qblocks, G;
+  int causal;
+  int k;                                  // round of the dealing
+  int nb, hk, part, b, iters, mb_first, per_head;
+  __device__ explicit BwdItems(const ItbAttnArgs& a) {
+    nparts = a.bwd_parts > 1 ? a.bwd_parts : 1;
+    width = a.KV * nparts;
+    n_qblocks = (a.T + 127) / 128;
+    total = n_qblocks * width * a.B;
+    G = a.H / a.KV;
+    causal = a.causal;
+    B = a.B;
+    k = -1;
+  }
+  // the next item of this CTA that has tiles
+  __device__ bool next() {
+    for (;;) {
+      ++k;
+      const int base = k * static_cast<int>(gridDim.x);
+      if (base >= total) return false;
+      const int i = base + static_cast<int>((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+      if (i >= total) continue;
+      nb = i / (width * B);
+      const int r = i % (width * B);
+      b = r / width;
+      hk = (r % width) / nparts;
+      part = r % nparts;
+      mb_first = causal ? nb : 0;
+      per_head = n_qblocks - mb_first;
+      const int pairs = per_head * G;
+      iters = pairs > part ? (pairs - part + nparts - 1) / nparts : 0;
+      if (iters > 0) return true;
+    }
+  }
+  __device__ void tile(int it, int& h, int& mb) const {
+    const int g = part + it * nparts;
+    h = hk * G + g / per_head;
+    mb = mb_first + g % per_head;
+  }
+  int B;
+};
+
+// Persistent: one CTA per SM; the next item's loads, S and dP run under the last tiles of the one before.  Tiles
+// and items are numbered through (n, c), which gives every barrier its parity.
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const __grid_constant__ CUtensorMap tdq, const ItbAttnArgs a, int* err) {
   using Cfg = BwdCfg<D>;
-  constexpr int S = Cfg::kQStages;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  constexpr int SO = Cfg::kdOStages;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  // the swizzled tiles need a 1024-byte boundary; there is no room left to round up at head size 128
+  if (smem_u32(smem) & 1023) {
+    if (threadIdx.x == 0) atomicCAS(err, 0, 200);
+    return;
+  }
   float* s_lse = reinterpret_cast<float*>(smem + Cfg::kOffStat);
   float* s_delta = s_lse + 2 * 128;
+  constexpr int SK = Cfg::kKvStages;
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
-  uint64_t* q_full = kv_full + 1;
+  uint64_t* kv_empty = kv_full + 2;
+  uint64_t* q_full = kv_empty + 2;      // Q tile and the statistics of its rows
   uint64_t* q_empty = q_full + 2;
-  uint64_t* s_full = q_empty + 2;
-  uint64_t* p_full = s_full + 1;
-  uint64_t* dq_full = p_full + 1;
+  uint64_t* do_full = q_empty + 2;
+  uint64_t* do_empty = do_full + 2;
+  uint64_t* s_full = do_empty + 2;
+  uint64_t* dp_full = s_full + 1;
+  uint64_t* p_full = dp_full + 1;
+  uint64_t* ds_full = p_full + 1;
+  uint64_t* dq_full = ds_full + 1;
   uint64_t* dq_drained = dq_full + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(dq_drained + 1);
+  uint64_t* acc_full = dq_drained + 1;      // dK and dV of an item
+  uint64_t* acc_drained = acc_full + 1;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_drained + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // The (query head of the group, query tile) pairs that meet this CTA's 128 keys are dealt out to
-  // `nparts` CTAs in turn (a.bwd_parts > 1 when the plain grid would leave most SMs idle: few key
-  // tiles, one KV head per rank under tensor parallelism); each then adds its dK / dV into fp32
-  // accumulators instead of writing them.
-  const int nparts = a.bwd_parts > 1 ? a.bwd_parts : 1;
-  const int nb = blockIdx.x, hk = blockIdx.y / nparts, part = blockIdx.y % nparts, b = blockIdx.z;
-  const int G = a.H / a.KV;
-  const int n0 = nb * 128;
-  const int n_qblocks = (a.T + 127) / 128;
-  const int mb_first = a.causal ? nb : 0;
-  const int per_head = n_qblocks - mb_first;
-  const int total_iters = per_head * G;
-  const int iters = total_iters > part ? (total_iters - part + nparts - 1) / nparts : 0;
-  auto tile_of = [&](int it, int& h, int& mb) {
-    const int g = part + it * nparts;
-    h = hk * G + g / per_head;
-    mb = mb_first + g % per_head;
-  };
+  const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&q_full[s], 1);
+      mbar_init(&kv_full[s], 1);
+      mbar_init(&kv_empty[s], 1);
+      mbar_init(&q_full[s], 2);
       mbar_init(&q_empty[s], 1);
+      mbar_init(&do_full[s], 1);
+      mbar_init(&do_empty[s], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(p_full, kSoftmaxThreads);
+    mbar_init(dp_full, 1);
+    mbar_init(p_full, 8);
+    mbar_init(ds_full, 8);
     mbar_init(dq_full, 1);
-    mbar_init(dq_drained, kSoftmaxThreads / 32);
+    mbar_init(dq_drained, 4);
+    mbar_init(acc_full, 1);
+    mbar_init(acc_drained, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
+  if (warp == 13) {
     tmem_alloc(tmem_holder, 512);
     tmem_relinquish();
   }
@@ -142,297 +222,429 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_holder;
   const uint32_t tm_S = tmem_base, tm_dP = tmem_base + 128, tm_dV = tmem_base + 256, tm_dK = tmem_base + 256 + D;
-  constexpr bool kAlias = D > 64;     // no TMEM columns left for dQ: it goes over the spent S^T
-  const uint32_t tm_dQ = kAlias ? tmem_base : tmem_base + 256 + 2 * D;
+  constexpr bool kAlias = D > 64;     // no TMEM columns left for dQ: it goes over the spent dP^T
+  const uint32_t tm_dQ = kAlias ? tm_dP : tmem_base + 256 + 2 * D;
+  // with columns to spare dS^T goes to TMEM too, as dK's operand: 32 KB less to read from shared memory a tile
+  constexpr bool kTmemdS = !kAlias;
+  const uint32_t tm_dS = tmem_base + 256 + 3 * D;
+  auto give_up = [&](int code) {
+    atomicCAS(err, 0, code);
+    *abort_flag = 1;
+  };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return warp_wait(bar, parity & 1, abort_flag); };
+  BwdItems item(a);
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tq);
-      tma_prefetch_desc(&tk);
-      tma_prefetch_desc(&tv);
-      tma_prefetch_desc(&tdo);
-      mbar_expect_tx(kv_full, 2 * Cfg::kTile);
-#pragma unroll
-      for (int at = 0; at < Cfg::kAtoms; ++at) {
-        tma_load_3d(smem + Cfg::kOffK + at * kAtom, &tk, kv_full, hk * D + at * 64, n0, b);
-        tma_load_3d(smem + Cfg::kOffV + at * kAtom, &tv, kv_full, hk * D + at * 64, n0, b);
-      }
-      for (int it = 0; it < iters; ++it) {
-        const int st = it % S;
-        const uint32_t ph = (it / S) & 1;
-        if (!mbar_wait(&q_empty[st], ph ^ 1) || *abort_flag) {
-          atomicCAS(err, 0, 201);
-          *abort_flag = 1;
-          break;
-        }
-        int h, mb;
-        tile_of(it, h, mb);
-        mbar_expect_tx(&q_full[st], 2 * Cfg::kTile);
-#pragma unroll
-        for (int at = 0; at < Cfg::kAtoms; ++at) {
-          tma_load_3d(smem + Cfg::kOffQ + st * Cfg::kTile + at * kAtom, &tq, &q_full[st], h * D + at * 64, mb * 128, b);
-          tma_load_3d(smem + Cfg::kOffdO + st * Cfg::kTile + at * kAtom, &tdo, &q_full[st], h * D + at * 64, mb * 128,
-                      b);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t id_s = make_idesc_bf16_f32(128, 128, false, false);
-    constexpr uint32_t id_kv = make_idesc_bf16_f32(128, D, false, true);
-    constexpr uint32_t id_q = make_idesc_bf16_f32(128, D, true, true);
-    const uint32_t aK = smem_u32(smem + Cfg::kOffK), aV = smem_u32(smem + Cfg::kOffV);
-    const uint32_t aP = smem_u32(smem + Cfg::kOffP), adS = smem_u32(smem + Cfg::kOffdS);
-    // Shared-memory descriptors are built once; a k-step only adds its byte offset (>> 4) to them.
-    const uint64_t dK_k = make_smem_desc_sw128(aK, 16, 1024), dV_k = make_smem_desc_sw128(aV, 16, 1024);
-    const uint64_t dP_k = make_smem_desc_sw128(aP, 16, 1024), ddS_k = make_smem_desc_sw128(adS, 16, 1024);
-    const uint64_t ddS_m = make_smem_desc_sw128(adS, kAtom, 1024), dK_m = make_smem_desc_sw128(aK, kAtom, 1024);
-    const uint32_t aQ0 = smem_u32(smem + Cfg::kOffQ), adO0 = smem_u32(smem + Cfg::kOffdO);
-    const uint64_t dQ_k0 = make_smem_desc_sw128(aQ0, 16, 1024), ddO_k0 = make_smem_desc_sw128(adO0, 16, 1024);
-    const uint64_t dQ_m0 = make_smem_desc_sw128(aQ0, kAtom, 1024), ddO_m0 = make_smem_desc_sw128(adO0, kAtom, 1024);
-    constexpr uint64_t kStageStep = (S > 1 ? Cfg::kTile : 0) >> 4;
-    bool ok = mbar_wait(kv_full, 0);
-    if (!ok && lane == 0) atomicCAS(err, 0, 202);
-    auto issue_scores = [&](int it) {     // S^T and dP^T of tile `it`
-      const int st = it % S;
-      if (!mbar_wait(&q_full[st], (it / S) & 1) || *abort_flag) return false;
-      // with aliasing, dQ of the previous tile sits over S^T until the softmax warps have read it out
-      if (kAlias && it > 0 && (!mbar_wait(dq_drained, (it - 1) & 1) || *abort_flag)) return false;
-      tc_fence_after_sync();
+  // 512 threads of 128 registers at the launch, 128 x (2 x 144 + 168 + 56) after the split
+  if (warp >= 12) {
+    regs_shrink<56>();
+    if (warp == 12) {
+      // ---------------------------------------------------------------- TMA producer
       if (lane == 0) {
-        const uint64_t dQ_k = dQ_k0 + st * kStageStep, ddO_k = ddO_k0 + st * kStageStep;
+        tma_prefetch_desc(&tq);
+        tma_prefetch_desc(&tk);
+        tma_prefetch_desc(&tv);
+        tma_prefetch_desc(&tdo);
+      }
+      bool ok = true;
+      uint32_t n = 0;
+      for (uint32_t c = 0; ok && item.next(); ++c) {
+        const int sk = c % SK;
+        ok = wait(&kv_empty[sk], c / SK + 1);
+        if (!ok) break;
+        if (lane == 0) {
+          uint8_t* kv = smem + Cfg::kOffK + sk * 2 * Cfg::kTile;
+          mbar_expect_tx(&kv_full[sk], 2 * Cfg::kTile);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint64_t off = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;
-          umma_f16_ss(tm_S, dK_k + off, dQ_k + off, id_s, kk > 0);
+          for (int at = 0; at < Cfg::kAtoms; ++at) {
+            tma_load_3d(kv + at * kAtom, &tk, &kv_full[sk], item.hk * D + at * 64, item.nb * 128, item.b);
+            tma_load_3d(kv + Cfg::kTile + at * kAtom, &tv, &kv_full[sk], item.hk * D + at * 64, item.nb * 128, item.b);
+          }
         }
+        for (int it = 0; it < item.iters; ++it, ++n) {
+          const int st = n & 1, so = n % SO;
+          int h, mb;
+          item.tile(it, h, mb);
+          // statistics of four query rows per lane, in flight under the wait; rows beyond the sequence get
+          // probability 0 (lse = +inf) and delta 0
+          float lse4[4], delta4[4];
+          const long long so_row = (static_cast<long long>(item.b) * a.H + h) * a.T;
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint64_t off = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;
-          umma_f16_ss(tm_dP, dV_k + off, ddO_k + off, id_s, kk > 0);
-        }
-        umma_commit(s_full);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (ok && iters > 0 && !issue_scores(0)) {
-      if (lane == 0) atomicCAS(err, 0, 203);
-      ok = false;
-    }
-    for (int it = 0; it < iters && ok; ++it) {
-      const int st = it % S;
-      ok = mbar_wait(p_full, it & 1) && !*abort_flag;
-      // its own dQ columns are rewritten below: the previous tile's dQ must have been read out
-      if (ok && !kAlias && it > 0) ok = mbar_wait(dq_drained, (it - 1) & 1) && !*abort_flag;
-      if (!ok) {
-        if (lane == 0) atomicCAS(err, 0, 204);
-        break;
-      }
-      tc_fence_after_sync();
-      if (lane == 0) {
-        const uint64_t dQ_m = dQ_m0 + st * kStageStep, ddO_m = ddO_m0 + st * kStageStep;
+          for (int r = 0; r < 4; ++r) {
+            const int qrow = mb * 128 + r * 32 + lane;
+            lse4[r] = qrow < a.T ? __ldg(a.lse + so_row + qrow) * kLog2e : INFINITY;
+            delta4[r] = qrow < a.T ? __ldg(a.delta + so_row + qrow) : 0.f;
+          }
+          ok = wait(&q_empty[st], (n >> 1) + 1);
+          if (!ok) break;
+          if (lane == 0) {
+            mbar_expect_tx(&q_full[st], Cfg::kTile);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {       // contraction over the 128 query rows of the tile
-          const uint64_t koff = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;   // K-major operand: P^T / dS^T
-          const uint64_t moff = (kk * 2048) >> 4;                            // MN-major operand: 16 rows down
-          umma_f16_ss(tm_dV, dP_k + koff, ddO_m + moff, id_kv, (it > 0 || kk > 0));
-          umma_f16_ss(tm_dK, ddS_k + koff, dQ_m + moff, id_kv, (it > 0 || kk > 0));
-        }
+            for (int at = 0; at < Cfg::kAtoms; ++at)
+              tma_load_3d(smem + Cfg::kOffQ + st * Cfg::kTile + at * kAtom, &tq, &q_full[st], h * D + at * 64, mb * 128,
+                          item.b);
+          }
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {       // contraction over the 128 keys
-          const uint64_t moff = (kk * 2048) >> 4;
-          umma_f16_ss(tm_dQ, ddS_m + moff, dK_m + moff, id_q, kk > 0);
-        }
-        umma_commit(&q_empty[st]);
-        umma_commit(dq_full);
-      }
-      __syncwarp();
-      if (it + 1 < iters && !issue_scores(it + 1)) {
-        if (lane == 0) atomicCAS(err, 0, 203);
-        ok = false;
-      }
-    }
-    if (!ok) *abort_flag = 1;
-  } else {
-    // ------------------------------------------------------------------ softmax / read-out warps
-    const int qd = warp & 3;
-    const int half = (warp - 2) >> 2;           // which half of the columns this warp takes
-    const int row = qd * 32 + lane;             // key row (softmax) and query row (dQ read-out)
-    const uint32_t lane_addr = static_cast<uint32_t>(qd * 32) << 16;
-    const int tid = (warp - 2) * 32 + lane;     // 0..255, for the per-tile statistics
-    const float sl2 = a.scale * kLog2e;
-    uint8_t* sP = smem + Cfg::kOffP;
-    uint8_t* sdS = smem + Cfg::kOffdS;
-    bool ok = true;
-    // lse * log2(e) (threads 0..127) or delta (threads 128..255) of query row tid & 127 of tile `it`;
-    // rows beyond the sequence get probability 0 (lse = +inf) and delta 0
-    auto load_stat = [&](int it) -> float {
-      int h, mb;
-      tile_of(it, h, mb);
-      const int qrow = mb * 128 + (tid & 127);
-      const long long so = (static_cast<long long>(b) * a.H + h) * a.T + qrow;
-      if (tid < 128) return qrow < a.T ? __ldg(a.lse + so) * kLog2e : INFINITY;
-      return qrow < a.T ? __ldg(a.delta + so) : 0.f;
-    };
-    float stat_next = iters > 0 ? load_stat(0) : 0.f;
-    for (int it = 0; it < iters; ++it) {
-      int h, mb;
-      tile_of(it, h, mb);
-      const int sb = it & 1;
-      // this tile's statistics were fetched while the previous tile was being processed
-      if (tid < 128)
-        s_lse[sb * 128 + tid] = stat_next;
-      else
-        s_delta[sb * 128 + tid - 128] = stat_next;
-      if (it + 1 < iters) stat_next = load_stat(it + 1);
-      softmax_warps_sync();
-      if (ok) {
-        ok = mbar_wait(s_full, it & 1) && !*abort_flag;
-        if (!ok) {
-          atomicCAS(err, 0, 205);
-          *abort_flag = 1;
+          for (int r = 0; r < 4; ++r) {
+            s_lse[st * 128 + r * 32 + lane] = lse4[r];
+            s_delta[st * 128 + r * 32 + lane] = delta4[r];
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&q_full[st]);
+          ok = wait(&do_empty[so], n / SO + 1);
+          if (!ok) break;
+          if (lane == 0) {
+            mbar_expect_tx(&do_full[so], Cfg::kTile);
+#pragma unroll
+            for (int at = 0; at < Cfg::kAtoms; ++at)
+              tma_load_3d(smem + Cfg::kOffdO + so * Cfg::kTile + at * kAtom, &tdo, &do_full[so], h * D + at * 64, mb * 128,
+                          item.b);
+          }
         }
       }
-      if (ok) {
+      if (!ok) give_up(201);
+    } else if (warp == 13) {
+      // ---------------------------------------------------------------- MMA issuer: one thread, elected per instruction
+      constexpr uint32_t id_s = make_idesc_bf16_f32(128, 128, false, false);
+      constexpr uint32_t id_kv = make_idesc_bf16_f32(128, D, false, true);
+      constexpr uint32_t id_q = make_idesc_bf16_f32(128, D, true, true);
+      const uint32_t aK = smem_u32(smem + Cfg::kOffK), aV = smem_u32(smem + Cfg::kOffV);
+      const uint32_t adS = smem_u32(smem + Cfg::kOffdS);
+      // Shared-memory descriptors are built once; a stage or k-step only adds its byte offset (>> 4) to them.
+      const uint64_t dK_k0 = make_smem_desc_sw128(aK, 16, 1024), dV_k0 = make_smem_desc_sw128(aV, 16, 1024);
+      const uint64_t ddS_k = make_smem_desc_sw128(adS, 16, 1024);
+      const uint64_t ddS_m = make_smem_desc_sw128(adS, kAtom, 1024), dK_m0 = make_smem_desc_sw128(aK, kAtom, 1024);
+      const uint32_t aQ0 = smem_u32(smem + Cfg::kOffQ), adO0 = smem_u32(smem + Cfg::kOffdO);
+      const uint64_t dQ_k0 = make_smem_desc_sw128(aQ0, 16, 1024), ddO_k0 = make_smem_desc_sw128(adO0, 16, 1024);
+      const uint64_t dQ_m0 = make_smem_desc_sw128(aQ0, kAtom, 1024), ddO_m0 = make_smem_desc_sw128(adO0, kAtom, 1024);
+      constexpr uint64_t kStageStep = Cfg::kTile >> 4, kKvStep = (2 * Cfg::kTile) >> 4;
+      auto wait_tc = [&](uint64_t* bar, uint32_t parity) {
+        const bool ok = wait(bar, parity);
         tc_fence_after_sync();
-        const bool key_ok = n0 + row < a.T;
-        // the mask matters on the diagonal tile and for the keys beyond the sequence only
-        const bool diag = a.causal && mb == nb;
-        const bool need_mask = diag || (n0 + 128 > a.T);
-        const float* lse = s_lse + sb * 128;
-        const float* dl = s_delta + sb * 128;
-#pragma unroll 1
-        for (int cg = 2 * half; cg < 2 * half + 2; ++cg) {
-          uint32_t rs[32], rp[32];
-          tmem_ld_32x32(tm_S + lane_addr + cg * 32, rs);
-          tmem_ld_32x32(tm_dP + lane_addr + cg * 32, rp);
+        return ok;
+      };
+      auto issue_s = [&](uint32_t c, uint32_t n) {       // S^T of tile n with item c's keys
+        const uint64_t dK_k = dK_k0 + (c % SK) * kKvStep, dQ_k = dQ_k0 + (n & 1) * kStageStep;
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint64_t off = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;
+          umma_f16_ss_elect(tm_S, dK_k + off, dQ_k + off, id_s, kk > 0);
+        }
+        umma_commit_elect(s_full);
+      };
+      auto issue_dp = [&](uint32_t c, uint32_t n) {
+        const uint64_t dV_k = dV_k0 + (c % SK) * kKvStep, ddO_k = ddO_k0 + (n % SO) * kStageStep;
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint64_t off = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;
+          umma_f16_ss_elect(tm_dP, dV_k + off, ddO_k + off, id_s, kk > 0);
+        }
+        umma_commit_elect(dp_full);
+      };
+      bool more = item.next(), ok = true;
+      uint32_t n = 0;
+      if (more) {
+        ok = wait_tc(&kv_full[0], 0) && wait_tc(&q_full[0], 0);
+        if (ok) {
+          issue_s(0, 0);
+          ok = wait_tc(&do_full[0], 0);
+          if (ok) issue_dp(0, 0);
+        }
+      }
+      for (uint32_t c = 0; more && ok; ++c) {
+        const int iters = item.iters;
+        more = item.next();
+        const uint64_t dK_m = dK_m0 + (c % SK) * kKvStep;
+        for (int it = 0; it < iters; ++it, ++n) {
+          const bool last = it + 1 == iters, next_tile = !last || more;
+          const uint32_t cn = last ? c + 1 : c;           // the next tile's item
+          ok = wait_tc(p_full, n);
+          if (ok && it == 0 && c > 0) ok = wait_tc(acc_drained, c - 1);
+          if (!ok) break;
+          const uint64_t ddO_m = ddO_m0 + (n % SO) * kStageStep;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)         // contraction over the 128 query rows of the tile
+            umma_f16_ts_elect(tm_dV, tm_S + (kk >> 2) * 64 + (kk & 3) * 8, ddO_m + ((kk * 2048) >> 4), id_kv,
+                              it > 0 || kk > 0);
+          umma_commit_elect(&do_empty[n % SO]);
+          auto next_s = [&]() {
+            bool got = true;
+            if (last) got = wait_tc(&kv_full[cn % SK], cn / SK);
+            if (got) got = wait_tc(&q_full[(n + 1) & 1], (n + 1) >> 1);
+            if (got) issue_s(cn, n + 1);
+            return got;
+          };
+          // a single stage of K and V is refilled only behind this tile's dQ
+          const bool early = !last || SK > 1;
+          if (next_tile && early) ok = next_s();
+          if (ok) ok = wait_tc(ds_full, n);
+          auto next_dp = [&]() {
+            bool got = wait_tc(&do_full[(n + 1) % SO], (n + 1) / SO);
+            if (got && kAlias) got = wait_tc(dq_drained, n);
+            if (got) issue_dp(cn, n + 1);
+            return got;
+          };
+          // dP of the next tile first where dQ does not need its columns: the softmax warps wait for it
+          if (ok && !kAlias && next_tile) ok = next_dp();
+          // its own columns: the previous tile's dQ must have been read out (at head size 128 dP waited for that)
+          if (ok && !kAlias && n > 0) ok = wait_tc(dq_drained, n - 1);
+          if (!ok) break;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {       // contraction over the 128 keys
+            const uint64_t moff = (kk * 2048) >> 4;                            // MN-major operand: 16 rows down
+            umma_f16_ss_elect(tm_dQ, ddS_m + moff, dK_m + moff, id_q, kk > 0);
+          }
+          umma_commit_elect(dq_full);
+          const uint64_t dQ_m = dQ_m0 + (n & 1) * kStageStep;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {       // contraction over the 128 query rows of the tile
+            const uint64_t koff = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;   // K-major operand
+            if constexpr (kTmemdS)
+              umma_f16_ts_elect(tm_dK, tm_dS + kk * 8, dQ_m + ((kk * 2048) >> 4), id_kv, it > 0 || kk > 0);
+            else
+              umma_f16_ss_elect(tm_dK, ddS_k + koff, dQ_m + ((kk * 2048) >> 4), id_kv, it > 0 || kk > 0);
+          }
+          umma_commit_elect(&q_empty[n & 1]);
+          if (last) {
+            umma_commit_elect(&kv_empty[c % SK]);
+            umma_commit_elect(acc_full);
+          }
+          if (kAlias && next_tile) {
+            if (!early) ok = next_s();
+            if (ok) ok = next_dp();
+            if (!ok) break;
+          }
+        }
+      }
+      if (!ok) give_up(204);
+    }
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------------ dQ read-out: query row = TMEM lane
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const bool issuer = warp == 8 && lane == 0;
+    regs_grow<168>();
+    bool ok = true;       // a warp that gave up keeps meeting the others at the barriers
+    uint32_t n = 0;
+    while (item.next()) {
+      for (int it = 0; it < item.iters; ++it, ++n) {
+        int h, mb;
+        item.tile(it, h, mb);
+        if (ok) {
+          ok = wait(dq_full, n);
+          if (!ok) give_up(206);
+        }
+        tc_fence_after_sync();
+        // All columns into registers, so that the tensor core gets them back at once; then 64 columns a round through
+        // two fp32 staging blocks of 32 columns (128-byte swizzle), one bulk add-reduction each.
+        uint32_t r[D / 32][32];
+        if (ok) {
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) tmem_ld_32x32(tm_dQ + lane_addr + c * 32, r[c]);
           tmem_ld_wait();
-          float pv[32], dv[32];
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_drained);
+        }
+#pragma unroll
+        for (int round = 0; round < D / 64; ++round) {
+          if (issuer) tma_store_wait_read<0>();     // the blocks have been read
+          readout_warps_sync();
+          if (ok) {
+#pragma unroll
+            for (int blk = 0; blk < 2; ++blk) {
+              uint8_t* dst = smem + Cfg::kOffStage + blk * kAtom + row * 128;
+              const uint32_t(&v)[32] = r[round * 2 + blk];
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<float4*>(dst + ((j ^ (row & 7)) << 4)) =
+                    make_float4(__uint_as_float(v[4 * j]) * a.scale, __uint_as_float(v[4 * j + 1]) * a.scale,
+                                __uint_as_float(v[4 * j + 2]) * a.scale, __uint_as_float(v[4 * j + 3]) * a.scale);
+            }
+          }
+          fence_proxy_async_smem();
+          readout_warps_sync();
+          if (issuer && ok) {
+            tma_reduce_add_3d(&tdq, smem + Cfg::kOffStage, h * D + round * 64, mb * 128, item.b);
+            tma_reduce_add_3d(&tdq, smem + Cfg::kOffStage + kAtom, h * D + round * 64 + 32, mb * 128, item.b);
+            tma_store_commit();
+          }
+        }
+      }
+    }
+    if (issuer) tma_store_wait<0>();
+  } else {
+    // ------------------------------------------------------------------ softmax: key row = TMEM lane
+    regs_grow<144>();
+    const int half = warp >> 2;                 // which half of the query columns this warp takes
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const float sl2 = a.scale * kLog2e;
+    bool ok = true;
+    uint32_t n = 0;
+    for (uint32_t c = 0; ok && item.next(); ++c) {
+      const int n0 = item.nb * 128, krow = n0 + row;
+      const bool key_ok = krow < a.T;
+      for (int it = 0; it < item.iters; ++it, ++n) {
+        int h, mb;
+        item.tile(it, h, mb);
+        const int st = n & 1;
+        ok = wait(s_full, n);
+        if (!ok) break;
+        tc_fence_after_sync();
+        uint32_t rs[2][32];
+        tmem_ld_32x32(tm_S + lane_addr + half * 64, rs[0]);
+        tmem_ld_32x32(tm_S + lane_addr + half * 64 + 32, rs[1]);
+        ok = wait(&q_full[st], n >> 1);      // the statistics have been written (S waited for the tile itself)
+        tmem_ld_wait();
+        if (!ok) break;
+        // the mask matters on the diagonal tile and for the keys beyond the sequence only
+        const bool diag = a.causal && mb == item.nb;
+        const bool need_mask = diag || (n0 + 128 > a.T);
+        const float* lse = s_lse + st * 128 + half * 64;
+        const float* dl = s_delta + st * 128 + half * 64;
+        float p[64];
+#pragma unroll
+        for (int cg = 0; cg < 2; ++cg) {
 #pragma unroll
           for (int j4 = 0; j4 < 32; j4 += 4) {
             const float4 l4 = *reinterpret_cast<const float4*>(lse + cg * 32 + j4);
-            const float4 d4 = *reinterpret_cast<const float4*>(dl + cg * 32 + j4);
-            const float lv[4] = {l4.x, l4.y, l4.z, l4.w}, dd[4] = {d4.x, d4.y, d4.z, d4.w};
+            const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int j = j4 + e, m = cg * 32 + j;
-              float p = ex2(fmaf(__uint_as_float(rs[j]), sl2, -lv[e]));
-              if (need_mask && (!key_ok || (diag && row > m))) p = 0.f;
-              pv[j] = p;
-              dv[j] = p * (__uint_as_float(rp[j]) - dd[e]);
-            }
+            for (int e = 0; e < 4; ++e) p[cg * 32 + j4 + e] = ex2(fmaf(__uint_as_float(rs[cg][j4 + e]), sl2, -lv[e]));
           }
-          uint8_t* rowP = sP + (cg >> 1) * kAtom + row * 128;
-          uint8_t* rowS = sdS + (cg >> 1) * kAtom + row * 128;
+          if (need_mask) {
 #pragma unroll
-          for (int c8 = 0; c8 < 4; ++c8) {
-            const int pos = (((cg & 1) << 2) + c8) ^ (row & 7);
-            *reinterpret_cast<uint4*>(rowP + pos * 16) = pack8(&pv[c8 * 8]);
-            *reinterpret_cast<uint4*>(rowS + pos * 16) = pack8(&dv[c8 * 8]);
+            for (int j = 0; j < 32; ++j)
+              if (!key_ok || (diag && row > half * 64 + cg * 32 + j)) p[cg * 32 + j] = 0.f;
           }
+          uint32_t w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) w[j] = pack2(p[cg * 32 + 2 * j], p[cg * 32 + 2 * j + 1]);
+          // over the first half of the columns that this warp alone has read
+          tmem_st_32x16(tm_S + lane_addr + half * 64 + cg * 16, w);
         }
-        fence_proxy_async_smem();
+        tmem_st_wait();
         tc_fence_before_sync();
-        mbar_arrive(p_full);
-        ok = mbar_wait(dq_full, it & 1) && !*abort_flag;
-        if (!ok) {
-          atomicCAS(err, 0, 206);
-          *abort_flag = 1;
-        }
-      }
-      if (ok) {
-        // dQ of the tile: TMEM -> fp32 staging over the spent P^T / dS^T buffers (32 columns per
-        // 16 KB block, 128-byte swizzle) -> one bulk add-reduction per block into the fp32 dQ buffer
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+        ok = wait(dp_full, n);
+        if (!ok) break;
         tc_fence_after_sync();
-#pragma unroll 1
-        for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(tm_dQ + lane_addr + c * 32, r);
-          tmem_ld_wait();
-          uint8_t* dst = smem + Cfg::kOffP + c * kAtom + row * 128;
+        tmem_ld_32x32(tm_dP + lane_addr + half * 64, rs[0]);
+        tmem_ld_32x32(tm_dP + lane_addr + half * 64 + 32, rs[1]);
+        // dS of the tile before has been read; at head size 128 dp_full says so
+        if (!kAlias && n > 0) ok = wait(&q_empty[(n - 1) & 1], (n - 1) >> 1);
+        tmem_ld_wait();
+        if (!ok) break;
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(dst + ((j ^ (row & 7)) << 4)) =
-                make_float4(__uint_as_float(r[4 * j]) * a.scale, __uint_as_float(r[4 * j + 1]) * a.scale,
-                            __uint_as_float(r[4 * j + 2]) * a.scale, __uint_as_float(r[4 * j + 3]) * a.scale);
+        for (int cg = 0; cg < 2; ++cg) {
+          const uint32_t(&rp)[32] = rs[cg];
+          uint8_t* rowS = smem + Cfg::kOffdS + half * kAtom + row * 128;
+          uint32_t w[16];
+#pragma unroll
+          for (int j4 = 0; j4 < 32; j4 += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(dl + cg * 32 + j4);
+            const float* pj = &p[cg * 32 + j4];
+            w[j4 / 2] = pack2(pj[0] * (__uint_as_float(rp[j4]) - d4.x), pj[1] * (__uint_as_float(rp[j4 + 1]) - d4.y));
+            w[j4 / 2 + 1] =
+                pack2(pj[2] * (__uint_as_float(rp[j4 + 2]) - d4.z), pj[3] * (__uint_as_float(rp[j4 + 3]) - d4.w));
+          }
+#pragma unroll
+          for (int c8 = 0; c8 < 4; ++c8)
+            *reinterpret_cast<uint4*>(rowS + (((cg * 4 + c8) ^ (row & 7)) << 4)) =
+                make_uint4(w[4 * c8], w[4 * c8 + 1], w[4 * c8 + 2], w[4 * c8 + 3]);
+          if constexpr (kTmemdS) tmem_st_32x16(tm_dS + lane_addr + half * 32 + cg * 16, w);
         }
+        if constexpr (kTmemdS) tmem_st_wait();
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(dq_drained);
+        if (lane == 0) mbar_arrive(ds_full);
       }
-      softmax_warps_sync();     // every row of the staging blocks is written
-      if (ok && tid == 0) {
+      if (ok) ok = wait(acc_full, c);
+      if (!ok) break;
+      tc_fence_after_sync();
+      // dK (scaled) and dV of the item's 128 keys; a warp has 32 rows and half of the columns.  As bf16 they go through
+      // the warp's part of the spent dS^T, so that neighbouring lanes write neighbouring 16 bytes: with a row per
+      // lane each store touched 32 lines, 5000 cycles an item at head size 64.
+      if (item.nparts == 1) {
+        constexpr int kLanes = D / 16;           // lanes per row
+        uint8_t* mine = smem + Cfg::kOffdS + warp * 4096;
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c)
-          tma_reduce_add_3d(&tdq, smem + Cfg::kOffP + c * kAtom, h * D + c * 32, mb * 128, b);
-        tma_store_commit();
-        // the staging blocks are P^T / dS^T again after the barrier at the top of the next tile
-        tma_store_wait_read<0>();
-      }
-    }
-    if (tid == 0) tma_store_wait<0>();
-    if (ok && iters > 0 && nparts > 1) {
-      // this CTA's share of dK (scaled) and dV: added to the fp32 accumulators [2][B, T, KV, D]
-      const int krow = n0 + row;
-      const long long plane = static_cast<long long>(a.B) * a.T * a.KV * D;
-      float* dka = a.dkv_accum + ((static_cast<long long>(b) * a.T + krow) * a.KV + hk) * D;
-      float* dva = dka + plane;
-#pragma unroll 1
-      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-        uint32_t rk[32], rv[32];
-        tmem_ld_32x32(tm_dK + lane_addr + c * 32, rk);
-        tmem_ld_32x32(tm_dV + lane_addr + c * 32, rv);
-        tmem_ld_wait();
-        if (krow < a.T) {
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t tm = (which ? tm_dV : tm_dK) + lane_addr + half * (D / 2);
+          const float f = which ? 1.f : a.scale;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dka + c * 32 + j),
-                         "f"(__uint_as_float(rk[j]) * a.scale), "f"(__uint_as_float(rk[j + 1]) * a.scale),
-                         "f"(__uint_as_float(rk[j + 2]) * a.scale), "f"(__uint_as_float(rk[j + 3]) * a.scale)
-                         : "memory");
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dva + c * 32 + j),
-                         "f"(__uint_as_float(rv[j])), "f"(__uint_as_float(rv[j + 1])), "f"(__uint_as_float(rv[j + 2])),
-                         "f"(__uint_as_float(rv[j + 3]))
-                         : "memory");
+          for (int cc = 0; cc < D / 64; ++cc) {
+            uint32_t r[32];
+            tmem_ld_32x32(tm + cc * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float v[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]) * f;
+              // 16-byte pieces of a row in an order that keeps the lanes on different banks
+              *reinterpret_cast<uint4*>(mine + lane * (D == 64 ? 64 : 128) +
+                                        (((cc * 4 + j) ^ (D == 64 ? (lane >> 1) & 3 : lane & 7)) << 4)) = pack8(v);
+            }
           }
+          if (which == 1) tc_fence_before_sync();
+          __syncwarp();
+          if (which == 1 && lane == 0) mbar_arrive(acc_drained);
+          __nv_bfloat16* base = static_cast<__nv_bfloat16*>(which ? a.dv : a.dk) +
+                                item.b * (which ? a.v_batch_stride : a.k_batch_stride) + item.hk * D + half * (D / 2);
+          const long long stride = which ? a.v_row_stride : a.k_row_stride;
+          const int piece = lane % kLanes;
+#pragma unroll
+          for (int i = 0; i < kLanes; ++i) {
+            const int rr = i * (32 / kLanes) + lane / kLanes, key = n0 + (warp & 3) * 32 + rr;
+            const uint4 v = *reinterpret_cast<const uint4*>(
+                mine + rr * (D == 64 ? 64 : 128) + ((piece ^ (D == 64 ? (rr >> 1) & 3 : rr & 7)) << 4));
+            if (key < a.T) *reinterpret_cast<uint4*>(base + key * stride + piece * 8) = v;
+          }
+          __syncwarp();
+        }
+      } else {
+        // this share's, added to the fp32 accumulators [2][B, T, KV, D]
+        const long long plane = static_cast<long long>(a.B) * a.T * a.KV * D;
+        float* dka = a.dkv_accum + ((static_cast<long long>(item.b) * a.T + krow) * a.KV + item.hk) * D;
+        float* dva = dka + plane;
+#pragma unroll
+        for (int i = 0; i < D / 64; ++i) {
+          const int cc = half * (D / 64) + i;
+          uint32_t rk[32], rv[32];
+          tmem_ld_32x32(tm_dK + lane_addr + cc * 32, rk);
+          tmem_ld_32x32(tm_dV + lane_addr + cc * 32, rv);
+          tmem_ld_wait();
+          if (i + 1 == D / 64) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_drained);
+          }
+          if (key_ok) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dka + cc * 32 + j),
+                           "f"(__uint_as_float(rk[j]) * a.scale), "f"(__uint_as_float(rk[j + 1]) * a.scale),
+                           "f"(__uint_as_float(rk[j + 2]) * a.scale), "f"(__uint_as_float(rk[j + 3]) * a.scale)
+                           : "memory");
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dva + cc * 32 + j),
+                           "f"(__uint_as_float(rv[j])), "f"(__uint_as_float(rv[j + 1])),
+                           "f"(__uint_as_float(rv[j + 2])), "f"(__uint_as_float(rv[j + 3]))
+                           : "memory");
+            }
+          }
+          __syncwarp();
         }
       }
-    } else if (ok && nparts == 1) {
-      // dK (scaled) and dV of this CTA's 128 keys; the last dq_full covered the MMAs that wrote them
-      const int krow = n0 + row;
-      __nv_bfloat16* dkg = static_cast<__nv_bfloat16*>(a.dk) + b * a.k_batch_stride +
-                           static_cast<long long>(krow) * a.k_row_stride + hk * D;
-      __nv_bfloat16* dvg = static_cast<__nv_bfloat16*>(a.dv) + b * a.v_batch_stride +
-                           static_cast<long long>(krow) * a.v_row_stride + hk * D;
-#pragma unroll 1
-      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-        uint32_t rk[32], rv[32];
-        tmem_ld_32x32(tm_dK + lane_addr + c * 32, rk);
-        tmem_ld_32x32(tm_dV + lane_addr + c * 32, rv);
-        tmem_ld_wait();
-        if (krow < a.T) {
-          float fk[32], fv[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            fk[j] = __uint_as_float(rk[j]) * a.scale;
-            fv[j] = __uint_as_float(rv[j]);
-          }
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            *reinterpret_cast<uint4*>(dkg + c * 32 + j) = pack8(&fk[j]);
-            *reinterpret_cast<uint4*>(dvg + c * 32 + j) = pack8(&fv[j]);
-          }
-        }
-      }
     }
+    if (!ok) give_up(205);
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 13) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
@@ -726,6 +938,13 @@ static int fwd_launch(const ItbAttnArgs* a, int* err, cudaStream_t s) {
   return static_cast<int>(cudaGetLastError());
 }
 
+// SMs of the current device: the grid of the persistent kernels.
+static cudaError_t sm_count(int* sms) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
+}
+
 __global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D) {
   // delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d]; D / 8 threads per (b,t,h), 16 bytes each
   const int tpr = D >> 3;                                        // threads per row: 8 or 16
@@ -805,7 +1024,7 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
   args.bwd_parts = args.dkv_accum ? itb_flash_attn_bwd_parts(args.B, args.T, args.H, args.KV, args.causal) : 1;
   const ItbAttnArgs* a = &args;
   using Cfg = BwdCfg<D>;
-  constexpr int smem = Cfg::kSmem + 1024;
+  constexpr int smem = Cfg::kSmem;
   static PerDeviceOnce configured;
   if (configured.first()) {
     cudaError_t e = cudaFuncSetAttribute(flash_bwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -833,8 +1052,12 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
     e = cudaMemsetAsync(a->dkv_accum, 0, kv_vecs * 4 * sizeof(float), s);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  dim3 grid((a->T + 127) / 128, a->KV * parts, a->B);
-  flash_bwd_tc_kernel<D><<<grid, kThreads, smem, s>>>(tq, tk, tv, tdo, tdq, *a, err);
+  int sms = 0;
+  e = sm_count(&sms);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long items = static_cast<long long>((a->T + 127) / 128) * a->KV * parts * a->B;
+  if (items > (1LL << 30)) return -5;      // items and their tiles are counted in 32 bits
+  flash_bwd_tc_kernel<D><<<static_cast<int>(items < sms ? items : sms), kThreads, smem, s>>>(tq, tk, tv, tdo, tdq, *a, err);
   const long long nvec = nrow * (D / 4);
   attn_dq_convert_tc_kernel<<<static_cast<int>((nvec + 255) / 256), 256, 0, s>>>(*a, D);
   if (parts > 1) attn_dkv_convert_tc_kernel<<<static_cast<int>((kv_vecs + 255) / 256), 256, 0, s>>>(*a, D);
@@ -844,16 +1067,19 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
 }  // namespace fatc
 }  // namespace itb
 
+// CTAs of one (key tile, KV head, batch).  The longest CTA (the first key tile: every query tile of every head of
+// the group) bounds the launch from below, so it is split until it is no longer than an even share of all tiles
+// and a little: one sequence of 2048 tokens with 8 KV heads of 4 query heads has 128 CTAs of up to 64 tiles, 29 a
+// SM.  Each share pays for fp32 accumulators (cleared, added to, converted), so no finer than that.
+// (1 x 2048 tokens, 32 / 8 heads of 64, the whole call: 159 us unsplit, 105 us in two shares.)
 extern "C" int itb_flash_attn_bwd_parts(int B, int T, int H, int KV, int causal) {
-  (void)causal;
-  const long long ctas = static_cast<long long>((T + 127) / 128) * KV * B;
-  const int sms = 148;
-  if (ctas <= 0 || ctas * 2 > sms) return 1;                 // at least half a wave as it is
-  const int most = ((T + 127) / 128) * (H / KV);             // tiles of the busiest CTA
-  int parts = static_cast<int>(sms / ctas);
-  if (parts > most) parts = most;
-  if (parts > 16) parts = 16;
-  return parts < 1 ? 1 : parts;
+  const long long nt = (T + 127) / 128, G = H / KV;
+  const long long most = nt * G;                             // tiles of the longest CTA
+  const long long tiles = (causal ? nt * (nt + 1) / 2 : nt * nt) * G * KV * B;
+  const long long share = tiles / 148 + tiles / (148 * 8) + 1;
+  int parts = 1;
+  while (parts < 16 && parts < most && (most + parts - 1) / parts > share) ++parts;
+  return parts;
 }
 
 extern "C" int itb_flash_attn_bwd_tc(const ItbAttnArgs* a, int* err, cudaStream_t s) {

@@ -168,12 +168,12 @@ typedef struct {
   float* delta;           // scratch [B, H, T] fp32
   float* dq_accum;        // scratch [B, T, H, D] fp32 (zeroed by the call)
   // tensor-core backward only, optional: scratch [2][B, T, KV, D] fp32 (zeroed by the call).  When it is
-  // there and the grid of one CTA per (key tile, KV head, batch) would fill less than half of the
-  // SMs, itb_flash_attn_bwd_parts() CTAs share each key tile and sum their dK / dV here.
+  // there, the work of a (key tile, KV head, batch) is split into itb_flash_attn_bwd_parts() shares that
+  // sum their dK / dV here.
   float* dkv_accum;
   int bwd_parts;          // set by the launcher
 } ItbAttnArgs;
-// How many CTAs the tensor-core backward puts on one (key tile, KV head, batch); 1 = the scratch
+// Into how many shares the tensor-core backward splits one (key tile, KV head, batch); 1 = the scratch
 // buffer `dkv_accum` is not needed.
 int itb_flash_attn_bwd_parts(int B, int T, int H, int KV, int causal);
 
