@@ -651,275 +651,372 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------ forward
-// One CTA owns 128 query rows of one head and walks over the 128-key tiles up to the diagonal:
-//   S[m,n] = Q[m,:] . K[n,:]     tcgen05.mma  Q (K-major) x K (K-major)          -> TMEM cols 0..127
-//   online softmax: one thread per query row reads its row of S from TMEM twice (maximum, then
-//   exponentials), so nothing crosses threads; P is written as bf16 in the swizzled operand layout
-//   O_j[m,d] = P[m,n] V[n,d]     tcgen05.mma  P (K-major) x V (MN-major)         -> TMEM cols 128..
-//   o = o * exp2(m_old - m_new) + O_j   in registers
-// 192 threads (TMA warp, MMA warp, 4 softmax warps) and 80 KB of shared memory at head size 64, so
-// two CTAs share an SM and one's tensor-core and TMA latencies hide behind the other's softmax.
+// One item is 256 query rows of one head, two tiles of 128, walking together over the 128-key tiles up to the
+// diagonal; per tile and step
+//   S[m,n] = Q[m,:] . K[n,:]     tcgen05.mma  Q (K-major) x K (K-major)          -> TMEM, 128 columns a tile
+//   online softmax: one thread per query row holds its row of S in registers, so nothing crosses threads;
+//   P goes as bf16 over the spent S in TMEM
+//   O[m,d] += P[m,n] V[n,d]      tcgen05.mma  P (from TMEM) x V (MN-major)       -> TMEM, D columns a tile
+// While four warps do the softmax of one tile, the tensor core works on the other.  O stays in TMEM: it is
+// multiplied by exp2(m_old - m_new) only when a row's maximum has grown by more than kGrowth since the last time,
+// until then P is taken relative to the older maximum (at most 2^kGrowth large; the final division is exact either
+// way).  Persistent, one CTA per SM; the next item's loads and first S run under the last steps of the one before.
+//
+// What bounds it: the exponentials, 16 per cycle and SM: 1024 cycles per 128 x 128 scores (head size 128: the two
+// contractions take as long).
+// Measured (causal): 16 x 1024 tokens, 12 heads of 64: 109 us with one tile per CTA, P through shared memory and O
+// added up in registers; 66 us now.  1 x 8192, 32 / 8 heads of 128: 1243 -> 437 us (1258 TFLOP/s, 0.77 of the
+// measured GEMM peak).  1 x 2048, 32 / 8 heads of 64: 80 -> 35 us.
 template <int D>
 struct FwdCfg {
   static constexpr int kAtoms = D / 64;
   static constexpr int kTile = kAtoms * kAtom;
-  static constexpr int kOffQ = 0;
-  static constexpr int kOffK = kTile;
-  static constexpr int kOffV = 2 * kTile;
-  static constexpr int kOffP = 3 * kTile;                 // [2 n-chunks][128 m][64 n]
-  static constexpr int kOffBar = kOffP + 2 * kAtom;
-  static constexpr int kSmem = kOffBar + 12 * 8 + 16;
-  static constexpr int kTmemCols = 256;
+  static constexpr int kStages = D == 64 ? 4 : 2;         // of K and of V
+  static constexpr int kOffQ = 0;                         // two tiles
+  static constexpr int kOffK = 2 * kTile;
+  static constexpr int kOffV = kOffK + kStages * kTile;
+  static constexpr int kOffOut = kOffV + kStages * kTile;   // 4 KB a softmax warp: O on its way out
+  static constexpr int kOffBar = kOffOut + 8 * 4096;
+  static constexpr int kSmem = kOffBar + (2 + 4 * kStages + 6) * 8 + 16;
+  static_assert(kSmem <= 232448, "shared memory of one SM");
 };
-constexpr int kFwdThreads = 192;
+constexpr int kFwdThreads = 320;     // 2 x 4 softmax warps, TMA warp, MMA warp
+constexpr float kGrowth = 8.f;
+
+struct FwdItems {
+  int pairs, HB, H, causal, n_blocks, T;
+  int k;
+  int m0, h, b;
+  int steps[2];                 // key tiles of the two query tiles; 0: the tile lies beyond the sequence
+  __device__ explicit FwdItems(const ItbAttnArgs& a) {
+    T = a.T;
+    H = a.H;
+    HB = a.H * a.B;
+    causal = a.causal;
+    n_blocks = (a.T + 127) / 128;
+    pairs = (n_blocks + 1) / 2;
+    k = -1;
+  }
+  // Items of later queries have more steps under a causal mask: longest first, dealt out to the CTAs to and fro.
+  __device__ bool next() {
+    for (;;) {
+      ++k;
+      const int base = k * static_cast<int>(gridDim.x);
+      if (base >= pairs * HB) return false;
+      const int i = base + static_cast<int>((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+      if (i >= pairs * HB) continue;
+      const int pair = pairs - 1 - i / HB, hb = i % HB;
+      h = hb % H;
+      b = hb / H;
+      m0 = pair * 256;
+      steps[0] = causal ? min(n_blocks, 2 * pair + 1) : n_blocks;
+      steps[1] = m0 + 128 >= T ? 0 : causal ? min(n_blocks, 2 * pair + 2) : n_blocks;
+      return true;
+    }
+  }
+};
 
 template <int D>
-__global__ void __launch_bounds__(kFwdThreads, D == 64 ? 2 : 1)
+__global__ void __launch_bounds__(kFwdThreads, 1)
 flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const ItbAttnArgs a, int* err) {
   using Cfg = FwdCfg<D>;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  constexpr int S = Cfg::kStages;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) {          // the swizzled tiles need a 1024-byte boundary
+    if (threadIdx.x == 0) atomicCAS(err, 0, 210);
+    return;
+  }
   uint64_t* q_full = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
-  uint64_t* k_full = q_full + 1;
-  uint64_t* k_empty = k_full + 1;
-  uint64_t* v_full = k_empty + 1;
-  uint64_t* v_empty = v_full + 1;
-  uint64_t* s_full = v_empty + 1;
-  uint64_t* p_full = s_full + 1;
-  uint64_t* o_full = p_full + 1;
-  uint64_t* o_drained = o_full + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_drained + 1);
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* k_full = q_empty + 1;
+  uint64_t* k_empty = k_full + S;
+  uint64_t* v_full = k_empty + S;
+  uint64_t* v_empty = v_full + S;
+  uint64_t* s_full = v_empty + S;       // one of each per query tile from here on
+  uint64_t* p_full = s_full + 2;
+  uint64_t* o_full = p_full + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heavier (later) query tiles first, so that the tail of the grid is made of short CTAs
-  const int mb = a.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hk = h / (a.H / a.KV);
-  const int m0 = mb * 128;
-  int n_blocks = (a.T + 127) / 128;
-  if (a.causal) n_blocks = min(n_blocks, mb + 1);
+  const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(k_full, 1);
-    mbar_init(k_empty, 1);
-    mbar_init(v_full, 1);
-    mbar_init(v_empty, 1);
-    mbar_init(s_full, 1);
-    mbar_init(p_full, 128);
-    mbar_init(o_full, 1);
-    mbar_init(o_drained, 4);
+    mbar_init(q_empty, 1);
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
+    }
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(&s_full[t], 1);
+      mbar_init(&p_full[t], 4);
+      mbar_init(&o_full[t], 1);
+    }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_holder, Cfg::kTmemCols);
+  if (warp == 9) {
+    tmem_alloc(tmem_holder, 512);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tm_S = tmem_base, tm_O = tmem_base + 128;
+  const uint32_t tm_S = tmem_base, tm_O = tmem_base + 256;     // tile t: S at + 128 t, O at + D t
+  auto give_up = [&](int code) {
+    atomicCAS(err, 0, code);
+    *abort_flag = 1;
+  };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return warp_wait(bar, parity & 1, abort_flag); };
+  FwdItems item(a);
 
-  if (warp == 0) {
+  if (warp == 8) {
+    // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tq);
       tma_prefetch_desc(&tk);
       tma_prefetch_desc(&tv);
-      mbar_expect_tx(q_full, Cfg::kTile);
+    }
+    bool ok = true;
+    uint32_t n = 0;                     // key tiles so far
+    for (uint32_t c = 0; ok && item.next(); ++c) {
+      const int hk = item.h / (a.H / a.KV);
+      ok = wait(q_empty, c + 1);
+      if (!ok) break;
+      if (lane == 0) {
+        mbar_expect_tx(q_full, 2 * Cfg::kTile);
 #pragma unroll
-      for (int at = 0; at < Cfg::kAtoms; ++at)
-        tma_load_3d(smem + Cfg::kOffQ + at * kAtom, &tq, q_full, h * D + at * 64, m0, b);
-      for (int j = 0; j < n_blocks; ++j) {
-        const uint32_t ph = j & 1;
-        if (!mbar_wait(k_empty, ph ^ 1) || *abort_flag) {
-          atomicCAS(err, 0, 211);
-          *abort_flag = 1;
-          break;
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int at = 0; at < Cfg::kAtoms; ++at)
+            tma_load_3d(smem + Cfg::kOffQ + t * Cfg::kTile + at * kAtom, &tq, q_full, item.h * D + at * 64,
+                        item.m0 + t * 128, item.b);
+      }
+      const int steps = max(item.steps[0], item.steps[1]);
+      for (int j = 0; j < steps; ++j, ++n) {
+        const int st = n % S;
+        ok = wait(&k_empty[st], n / S + 1);
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(&k_full[st], Cfg::kTile);
+#pragma unroll
+          for (int at = 0; at < Cfg::kAtoms; ++at)
+            tma_load_3d(smem + Cfg::kOffK + st * Cfg::kTile + at * kAtom, &tk, &k_full[st], hk * D + at * 64, j * 128, item.b);
         }
-        mbar_expect_tx(k_full, Cfg::kTile);
+        ok = wait(&v_empty[st], n / S + 1);
+        if (!ok) break;
+        if (lane == 0) {
+          mbar_expect_tx(&v_full[st], Cfg::kTile);
 #pragma unroll
-        for (int at = 0; at < Cfg::kAtoms; ++at)
-          tma_load_3d(smem + Cfg::kOffK + at * kAtom, &tk, k_full, hk * D + at * 64, j * 128, b);
-        if (!mbar_wait(v_empty, ph ^ 1) || *abort_flag) {
-          atomicCAS(err, 0, 212);
-          *abort_flag = 1;
-          break;
+          for (int at = 0; at < Cfg::kAtoms; ++at)
+            tma_load_3d(smem + Cfg::kOffV + st * Cfg::kTile + at * kAtom, &tv, &v_full[st], hk * D + at * 64, j * 128, item.b);
         }
-        mbar_expect_tx(v_full, Cfg::kTile);
-#pragma unroll
-        for (int at = 0; at < Cfg::kAtoms; ++at)
-          tma_load_3d(smem + Cfg::kOffV + at * kAtom, &tv, v_full, hk * D + at * 64, j * 128, b);
       }
     }
-  } else if (warp == 1) {
+    if (!ok) give_up(211);
+  } else if (warp == 9) {
+    // ------------------------------------------------------------------ MMA issuer: one thread, elected per instruction
     constexpr uint32_t id_s = make_idesc_bf16_f32(128, 128, false, false);
     constexpr uint32_t id_o = make_idesc_bf16_f32(128, D, false, true);
-    const uint32_t aQ = smem_u32(smem + Cfg::kOffQ), aK = smem_u32(smem + Cfg::kOffK);
-    const uint32_t aV = smem_u32(smem + Cfg::kOffV), aP = smem_u32(smem + Cfg::kOffP);
-    auto issue_scores = [&](int j) {
-      if (!mbar_wait(k_full, j & 1) || *abort_flag) return false;
+    constexpr uint64_t kStep = Cfg::kTile >> 4;
+    const uint64_t dQ0 = make_smem_desc_sw128(smem_u32(smem + Cfg::kOffQ), 16, 1024);
+    const uint64_t dK0 = make_smem_desc_sw128(smem_u32(smem + Cfg::kOffK), 16, 1024);
+    const uint64_t dV0 = make_smem_desc_sw128(smem_u32(smem + Cfg::kOffV), kAtom, 1024);
+    auto wait_tc = [&](uint64_t* bar, uint32_t parity) {
+      const bool ok = wait(bar, parity);
       tc_fence_after_sync();
-      if (lane == 0) {
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kAtom + (kk & 3) * 32;
-          umma_f16_ss(tm_S, make_smem_desc_sw128(aQ + off, 16, 1024), make_smem_desc_sw128(aK + off, 16, 1024), id_s,
-                      kk > 0);
-        }
-        umma_commit(k_empty);
-        umma_commit(s_full);
-      }
-      __syncwarp();
-      return true;
+      return ok;
     };
-    bool ok = mbar_wait(q_full, 0);
-    if (ok && n_blocks > 0) ok = issue_scores(0);
-    if (!ok && lane == 0) atomicCAS(err, 0, 213);
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      ok = mbar_wait(p_full, j & 1) && !*abort_flag;
-      if (ok && j > 0) ok = mbar_wait(o_drained, (j - 1) & 1) && !*abort_flag;
-      if (ok) ok = mbar_wait(v_full, j & 1) && !*abort_flag;
-      if (!ok) {
-        if (lane == 0) atomicCAS(err, 0, 214);
-        break;
-      }
-      tc_fence_after_sync();
-      if (lane == 0) {
+    auto issue_s = [&](int t, uint32_t n) {      // S of query tile t with the key tile numbered n
+      const uint64_t dQ = dQ0 + t * kStep, dK = dK0 + (n % S) * kStep;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {       // contraction over the 128 keys of the tile
-          const uint32_t koff = (kk >> 2) * kAtom + (kk & 3) * 32;
-          umma_f16_ss(tm_O, make_smem_desc_sw128(aP + koff, 16, 1024), make_smem_desc_sw128(aV + kk * 2048, kAtom, 1024),
-                      id_o, kk > 0);
-        }
-        umma_commit(v_empty);
-        umma_commit(o_full);
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint64_t off = ((kk >> 2) * kAtom + (kk & 3) * 32) >> 4;
+        umma_f16_ss_elect(tm_S + t * 128, dQ + off, dK + off, id_s, kk > 0);
       }
-      __syncwarp();
-      if (j + 1 < n_blocks && !issue_scores(j + 1)) {
-        if (lane == 0) atomicCAS(err, 0, 213);
-        ok = false;
-      }
-    }
-    if (!ok) *abort_flag = 1;
-  } else {
-    const int qd = warp & 3;
-    const int row = qd * 32 + lane;                 // query row of the tile
-    const uint32_t lane_addr = static_cast<uint32_t>(qd * 32) << 16;
-    const float sl2 = a.scale * kLog2e;
-    float o[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) o[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f;           // running maximum (scaled, log2 domain) and sum
-    uint8_t* rowP = smem + Cfg::kOffP + row * 128;
+      umma_commit_elect(&s_full[t]);
+    };
     bool ok = true;
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      ok = mbar_wait(s_full, j & 1) && !*abort_flag;
-      if (!ok) {
-        atomicCAS(err, 0, 215);
-        *abort_flag = 1;
-        break;
-      }
-      tc_fence_after_sync();
-      // only the diagonal tile and a ragged last tile need the mask
-      const bool masked = (a.causal && j == mb) || ((j + 1) * 128 > a.T);
-      const int n_lim = masked ? min(a.causal && j == mb ? row + 1 : 128, a.T - j * 128) : 128;   // keys [0, n_lim) visible
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tm_S + lane_addr + c * 32, r);
-        tmem_ld_wait();
-        if (!masked) {
+    uint32_t n0 = 0;                    // number of the item's first key tile
+    uint32_t np[2] = {0, 0};            // P tiles so far
+    for (uint32_t c = 0; ok && item.next(); ++c) {
+      const int steps = max(item.steps[0], item.steps[1]);
+      ok = wait_tc(q_full, c) && wait_tc(&k_full[n0 % S], n0 / S);
+      if (!ok) break;
+      // S of the item before has been read: its last P tiles were waited for
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
-        } else {
+      for (int t = 0; t < 2; ++t)
+        if (item.steps[t] > 0) issue_s(t, n0);
+      umma_commit_elect(&k_empty[n0 % S]);
+      if (steps == 1) umma_commit_elect(q_empty);
+      for (int j = 0; j < steps && ok; ++j) {
+        const uint32_t n = n0 + j;
+        const bool more_keys = j + 1 < steps;
+        ok = wait_tc(&v_full[n % S], n / S);
+        if (ok && more_keys) ok = wait_tc(&k_full[(n + 1) % S], (n + 1) / S);
+        const uint64_t dV = dV0 + (n % S) * kStep;
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i < n_lim) mx = fmaxf(mx, __uint_as_float(r[i]));
+        for (int t = 0; t < 2; ++t) {
+          if (!ok || j >= item.steps[t]) continue;
+          ok = wait_tc(&p_full[t], np[t]);
+          if (!ok) continue;
+          ++np[t];
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)       // contraction over the 128 keys of the tile
+            umma_f16_ts_elect(tm_O + t * D, tm_S + t * 128 + kk * 8, dV + ((kk * 2048) >> 4), id_o, j > 0 || kk > 0);
+          // S goes over this P: MMAs complete in the order of issue
+          if (j + 1 < item.steps[t])
+            issue_s(t, n + 1);
+          else
+            umma_commit_elect(&o_full[t]);
         }
+        if (!ok) break;
+        umma_commit_elect(&v_empty[n % S]);
+        if (more_keys) umma_commit_elect(&k_empty[(n + 1) % S]);
+        if (j + 2 == steps) umma_commit_elect(q_empty);
       }
-      mx *= sl2;      // sl2 > 0: scaling commutes with the maximum
-      const float m_new = fmaxf(m_run, mx);
-      // a row with no visible key so far keeps -inf: use 0 as the base so that exp2 yields 0, not NaN
-      const float base = m_new == -INFINITY ? 0.f : m_new;
-      const float corr = ex2(m_run - base);
-      float sum = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tm_S + lane_addr + c * 32, r);
-        tmem_ld_wait();
-        float pv[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float p = ex2(fmaf(__uint_as_float(r[i]), sl2, -base));
-          if (masked && c * 32 + i >= n_lim) p = 0.f;
-          pv[i] = p;
-          sum += p;
-        }
-        uint8_t* dst = rowP + (c >> 1) * kAtom;
-#pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8)
-          *reinterpret_cast<uint4*>(dst + (((((c & 1) << 2) + c8) ^ (row & 7)) << 4)) = pack8(&pv[c8 * 8]);
-      }
-      l_run = l_run * corr + sum;
-      m_run = m_new;
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      mbar_arrive(p_full);
-      ok = mbar_wait(o_full, j & 1) && !*abort_flag;
-      if (!ok) {
-        atomicCAS(err, 0, 216);
-        *abort_flag = 1;
-        break;
-      }
-      tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tm_O + lane_addr + c * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(o[c * 32 + i], corr, __uint_as_float(r[i]));
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(o_drained);
+      n0 += steps;
     }
-    const int qrow = m0 + row;
-    if (ok && qrow < a.T) {
+    if (!ok) give_up(213);
+  } else {
+    // ------------------------------------------------------------------ softmax: query row = TMEM lane
+    const int t = warp >> 2;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t tS = tm_S + t * 128 + lane_addr, tO = tm_O + t * D + lane_addr;
+    const float sl2 = a.scale * kLog2e;
+    bool ok = true;
+    uint32_t n = 0, items = 0;
+    while (ok && item.next()) {
+      const int steps = t ? item.steps[1] : item.steps[0], mb = item.m0 / 128 + t;
+      if (steps == 0) continue;
+      float base = 0.f;                 // what the exponents are relative to (scaled, log2 domain)
+      float l_run = 0.f;
+      for (int j = 0; j < steps; ++j, ++n) {
+        ok = wait(&s_full[t], n);
+        if (!ok) break;
+        tc_fence_after_sync();
+        uint32_t s[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(tS + c * 32, s[c]);
+        tmem_ld_wait();
+        // only the diagonal tile and a ragged last tile need the mask
+        const bool diag = a.causal && j == mb;
+        if (diag || (j + 1) * 128 > a.T) {
+          const int n_lim = min(diag ? row + 1 : 128, a.T - j * 128);   // keys [0, n_lim) visible
+#pragma unroll
+          for (int i = 0; i < 128; ++i)
+            if (i >= n_lim) s[i >> 5][i & 31] = __float_as_uint(-INFINITY);
+        }
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 128; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(s[i >> 5][i & 31]));
+        // sl2 > 0: scaling commutes with the maximum.  A row that has seen no key yet (l_run = 0) takes any finite
+        // maximum as its base, and 0 for none, so that exp2 yields 0, not NaN.
+        const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
+        const bool fresh = l_run == 0.f;
+        if (j == 0) {
+          base = mx == -INFINITY ? 0.f : mx;
+        } else if (__any_sync(~0u, fresh || mx > base + kGrowth)) {
+          const float new_base = fresh ? (mx == -INFINITY ? 0.f : mx) : fmaxf(base, mx);
+          const float corr = fresh ? 0.f : ex2(base - new_base);
+          l_run *= corr;
+          base = new_base;
+          // s_full says that the PV of the step before has completed
+#pragma unroll 1
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x16(tO + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            tmem_st_32x16(tO + c * 16, o);
+          }
+        }
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float p0 = ex2(fmaf(__uint_as_float(s[c][2 * i]), sl2, -base));
+            const float p1 = ex2(fmaf(__uint_as_float(s[c][2 * i + 1]), sl2, -base));
+            sum[(2 * i) & 3] += p0;
+            sum[(2 * i + 1) & 3] += p1;
+            w[i] = pack2(p0, p1);
+          }
+          tmem_st_32x16(tS + c * 16, w);
+        }
+        l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[t]);
+      }
+      if (ok) ok = wait(&o_full[t], items);
+      if (!ok) break;
+      ++items;
+      tc_fence_after_sync();
+      const int qrow = mb * 128 + row;
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.o) + b * a.o_batch_stride +
-                          static_cast<long long>(qrow) * a.o_row_stride + h * D;
+      // 64 columns of the warp's 32 rows at a time through shared memory, so that eight lanes write the 128 bytes
+      // of a row together
+      uint8_t* mine = smem + Cfg::kOffOut + warp * 4096;
 #pragma unroll
-      for (int i = 0; i < D; i += 8) {
-        float t[8];
+      for (int c = 0; c < D / 64; ++c) {
+        uint32_t r[2][32];
+        tmem_ld_32x32(tO + c * 64, r[0]);
+        tmem_ld_32x32(tO + c * 64 + 32, r[1]);
+        tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 8; ++e) t[e] = o[i + e] * inv;
-        *reinterpret_cast<uint4*>(op + i) = pack8(t);
+        for (int i = 0; i < 8; ++i) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[i >> 2][(i & 3) * 8 + e]) * inv;
+          *reinterpret_cast<uint4*>(mine + lane * 128 + ((i ^ (lane & 7)) << 4)) = pack8(v);
+        }
+        __syncwarp();
+        __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.o) + item.b * a.o_batch_stride + item.h * D + c * 64;
+        const int first = mb * 128 + (warp & 3) * 32;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3);
+          const uint4 v = *reinterpret_cast<const uint4*>(mine + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+          if (first + rr < a.T) *reinterpret_cast<uint4*>(op + (first + rr) * a.o_row_stride + (lane & 7) * 8) = v;
+        }
+        __syncwarp();
       }
-      a.lse[(static_cast<long long>(b) * a.H + h) * a.T + qrow] =
-          l_run > 0.f ? m_run * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
+      if (qrow < a.T)
+        a.lse[(static_cast<long long>(item.b) * a.H + item.h) * a.T + qrow] =
+            l_run > 0.f ? base * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
+      __syncwarp();
     }
+    if (!ok) give_up(215);
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 9) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(tmem_base, 512);
   }
+}
+
+// SMs of the current device: the grid of the persistent kernels.
+static cudaError_t sm_count(int* sms) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
 }
 
 template <int D>
 static int fwd_launch(const ItbAttnArgs* a, int* err, cudaStream_t s) {
   using Cfg = FwdCfg<D>;
-  constexpr int smem = Cfg::kSmem + 1024;
+  constexpr int smem = Cfg::kSmem;
   static PerDeviceOnce configured;
   if (configured.first()) {
     cudaError_t e = cudaFuncSetAttribute(flash_fwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -933,16 +1030,13 @@ static int fwd_launch(const ItbAttnArgs* a, int* err, cudaStream_t s) {
   if (!rc) rc = make_tmap_bf16_3d(&tv, a->v, static_cast<uint64_t>(a->KV) * D, a->T, a->B, a->v_row_stride,
                                   a->v_batch_stride, 64, 128);
   if (rc) return rc;
-  dim3 grid((a->T + 127) / 128, a->H, a->B);
-  flash_fwd_tc_kernel<D><<<grid, kFwdThreads, smem, s>>>(tq, tk, tv, *a, err);
+  int sms = 0;
+  const cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const long long items = static_cast<long long>(((a->T + 127) / 128 + 1) / 2) * a->H * a->B;
+  if (items > (1LL << 30)) return -5;      // counted in 32 bits
+  flash_fwd_tc_kernel<D><<<static_cast<int>(items < sms ? items : sms), kFwdThreads, smem, s>>>(tq, tk, tv, *a, err);
   return static_cast<int>(cudaGetLastError());
-}
-
-// SMs of the current device: the grid of the persistent kernels.
-static cudaError_t sm_count(int* sms) {
-  int device = 0;
-  const cudaError_t e = cudaGetDevice(&device);
-  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
 }
 
 __global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D) {
