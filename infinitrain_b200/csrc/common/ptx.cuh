@@ -88,6 +88,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// A wait of a whole warp: bounded, and all its lanes get the same answer.  The abort flag is looked at only while
+// there is something to wait for: a wait that finds its phase complete sits in the chain of every tile.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  for (uint32_t i = 0; i < kMbarPollLimit; ++i) {
+    if (__all_sync(~0u, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(~0u, *abort_flag != 0)) return false;
+    if (i > 64) __nanosleep(32);
+  }
+  return false;
+}
+
 // ---------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const void* desc) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(desc) : "memory");
@@ -345,12 +356,14 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+// for a whole, converged warp: one elected thread issues
+__device__ __forceinline__ void umma_f16_ss_pair_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                       uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
       :
       : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
@@ -365,9 +378,12 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t mbar_cluster_addr) {
 
 // One commit that arrives on the mbarrier at the same shared-memory offset in every CTA of `cta_mask`
 // (the pair: 0b11).  Signals only: no data moves, this is not a load.
-__device__ __forceinline__ void umma_commit_pair_mc(uint32_t mbar_addr, uint16_t cta_mask) {
+// For a whole, converged warp: one elected thread issues.
+__device__ __forceinline__ void umma_commit_pair_mc_elect(uint32_t mbar_addr, uint16_t cta_mask) {
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}\n" ::"r"(
           mbar_addr),
       "h"(cta_mask)
       : "memory");

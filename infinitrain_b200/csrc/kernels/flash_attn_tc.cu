@@ -72,17 +72,6 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return u;
 }
 
-// A wait of a whole warp: bounded, and all its lanes get the same answer.  The abort flag is looked at only while
-// there is something to wait for: a wait that finds its phase complete sits in the chain of every tile.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
-  for (uint32_t i = 0; i < kMbarPollLimit; ++i) {
-    if (__all_sync(~0u, mbar_try_wait(bar, parity))) return true;
-    if (__any_sync(~0u, *abort_flag != 0)) return false;
-    if (i > 64) __nanosleep(32);
-  }
-  return false;
-}
-
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -231,7 +220,7 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     atomicCAS(err, 0, code);
     *abort_flag = 1;
   };
-  auto wait = [&](uint64_t* bar, uint32_t parity) { return warp_wait(bar, parity & 1, abort_flag); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity & 1, abort_flag); };
   BwdItems item(a);
 
   // 512 threads of 128 registers at the launch, 128 x (2 x 144 + 168 + 56) after the split
@@ -771,7 +760,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     atomicCAS(err, 0, code);
     *abort_flag = 1;
   };
-  auto wait = [&](uint64_t* bar, uint32_t parity) { return warp_wait(bar, parity & 1, abort_flag); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity & 1, abort_flag); };
   FwdItems item(a);
 
   if (warp == 8) {
@@ -1167,6 +1156,7 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
 // SM.  Each share pays for fp32 accumulators (cleared, added to, converted), so no finer than that.
 // (1 x 2048 tokens, 32 / 8 heads of 64, the whole call: 159 us unsplit, 105 us in two shares.)
 extern "C" int itb_flash_attn_bwd_parts(int B, int T, int H, int KV, int causal) {
+  if (B <= 0 || T <= 0 || KV <= 0) return 1;
   const long long nt = (T + 127) / 128, G = H / KV;
   const long long most = nt * G;                             // tiles of the longest CTA
   const long long tiles = (causal ? nt * (nt + 1) / 2 : nt * nt) * G * KV * B;
