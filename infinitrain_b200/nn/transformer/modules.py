@@ -139,7 +139,7 @@ class MLP(Module):
             if _aligned():
                 y = self.c_proj(x1 * self.silu(x2))
                 return y if residual is None else y + residual
-            return self.c_proj(ops.swiglu(x1, x2), residual=residual)
+            return self.c_proj(ops.swiglu_pair(x1, x2), residual=residual)
         if _aligned():
             y = self.c_proj(self.gelu(self.c_fc(x)))
             return y if residual is None else y + residual

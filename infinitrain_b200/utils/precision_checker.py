@@ -222,6 +222,7 @@ class PrecisionChecker:
     # type exists there (src/autograd/*.cc); the fused ops have no finer-grained records
     _FUNCTION_NAMES = {"linear": "LinearFunction", "mlp_gelu": "MlpGeluFunction", "layernorm": "LayerNormFunction",
                        "rmsnorm": "RMSNormFunction", "gelu": "GeluFunction", "swiglu": "SwiGLUFunction",
+                       "swiglu_pair": "SwiGLUFunction",
                        "attention_packed": "AttentionFunction", "embedding": "EmbeddingFunction",
                        "cross_entropy": "CrossEntropyFunction"}
 

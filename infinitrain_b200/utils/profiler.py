@@ -110,8 +110,8 @@ class Profiler:
                         "adamw", "adam_advance", "sgd", "cast_into", "colsum", "flash_attn_fwd", "flash_attn_bwd",
                         "nvl_allreduce_scale", "nvl_rs_adamw_bcast", "nvl_ce_merge", "tp_gemm", "tp_wait")
     kCollectives = ("AllReduce", "AllGather", "ReduceScatter", "Send", "Recv", "BroadCast", "Barrier")
-    kForwardOps = ("linear", "mlp_gelu", "layernorm", "rmsnorm", "gelu", "swiglu", "swiglu_packed", "attention_packed",
-                   "embedding", "cross_entropy")
+    kForwardOps = ("linear", "mlp_gelu", "layernorm", "rmsnorm", "gelu", "swiglu", "swiglu_pair", "swiglu_packed",
+                   "attention_packed", "embedding", "cross_entropy")
 
     @staticmethod
     def _in_backward() -> bool:

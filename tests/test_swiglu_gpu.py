@@ -1,0 +1,35 @@
+"""The SwiGLU that reads its two inputs where they are, against the one that reads a copy: the same kernel, so the same
+bits, whatever the layout of the inputs and of the gradient."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _layouts(rows, F, dtype):
+    wide = torch.randn(rows, 2 * F + 24, device="cuda").to(dtype)
+    yield torch.randn(rows, F, device="cuda").to(dtype), torch.randn(rows, F, device="cuda").to(dtype)
+    yield wide[:, :F], wide[:, F:2 * F]                    # rows of one wider matrix
+    yield wide[:, 8:F + 8], torch.randn(rows, F, device="cuda").to(dtype)     # unequal row strides
+    yield wide[:, 1:F + 1], wide[:, F + 3:2 * F + 3]       # off the 16-byte boundary
+    yield torch.randn(F, rows, device="cuda").to(dtype).t(), wide[:, :F]      # columns contiguous
+    yield wide[:1, :F].expand(rows, F), wide[:, :F]        # one row for all
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,F", [(1, 8), (7, 264), (300, 1032)])
+def test_swiglu_pair_is_swiglu(rows, F, dtype):
+    from infinitrain_b200.ops import functional as ops
+
+    torch.manual_seed(rows)
+    for a, b in _layouts(rows, F, dtype):
+        for dout in (torch.randn(rows, F, device="cuda").to(dtype), torch.randn(F, rows, device="cuda").to(dtype).t(),
+                     torch.randn(rows, F + 1, device="cuda").to(dtype)[:, 1:]):
+            results = []
+            for fn in (ops.swiglu_pair, ops.swiglu):
+                x, y = a.detach().requires_grad_(), b.detach().requires_grad_()
+                out = fn(x, y)
+                # swiglu wants an aligned gradient (contiguous() leaves a single row where it is)
+                g = dout.clone(memory_format=torch.contiguous_format) if fn is ops.swiglu else dout
+                results.append((out, *torch.autograd.grad(out, (x, y), g)))
+            assert all(torch.equal(p, q) for p, q in zip(*results))
