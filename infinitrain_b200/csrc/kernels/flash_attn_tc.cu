@@ -99,8 +99,8 @@ struct BwdCfg {
 // (query head of the group, query tile) pairs that meet its keys.
 //
 // The pairs of one key tile and KV head are dealt out to `nparts` items in turn (a.bwd_parts > 1 when whole ones
-// would leave SMs idle: few key tiles, one KV head per rank under tensor parallelism); each then adds its dK / dV
-// into fp32 accumulators instead of writing them.  With a causal mask the items of the first keys have the most
+// would leave SMs idle: few key tiles, one KV head per rank under tensor parallelism); each then writes its dK / dV
+// to a slab of fp32 scratch of its own.  With a causal mask the items of the first keys have the most
 // tiles: items are ordered by that and dealt out to the CTAs to and fro, so that each gets about the same.
 struct BwdItems {
   int nparts, width, total, n_qblocks, G;
@@ -595,36 +595,34 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           __syncwarp();
         }
       } else {
-        // this share's, added to the fp32 accumulators [2][B, T, KV, D]
+        // this share's, into its own slab of the fp32 scratch [parts][2][B, T, KV, D]: the conversion adds the slabs up
+        // in order, so that the result does not depend on which share came first
         const long long plane = static_cast<long long>(a.B) * a.T * a.KV * D;
-        float* dka = a.dkv_accum + ((static_cast<long long>(item.b) * a.T + krow) * a.KV + item.hk) * D;
-        float* dva = dka + plane;
+        float* dks = a.dkv_accum + item.part * 2 * plane +
+                     ((static_cast<long long>(item.b) * a.T + krow) * a.KV + item.hk) * D + half * (D / 2);
 #pragma unroll
-        for (int i = 0; i < D / 64; ++i) {
-          const int cc = half * (D / 64) + i;
-          uint32_t rk[32], rv[32];
-          tmem_ld_32x32(tm_dK + lane_addr + cc * 32, rk);
-          tmem_ld_32x32(tm_dV + lane_addr + cc * 32, rv);
-          tmem_ld_wait();
-          if (i + 1 == D / 64) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_drained);
-          }
-          if (key_ok) {
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t tm = (which ? tm_dV : tm_dK) + lane_addr + half * (D / 2);
+          const float f = which ? 1.f : a.scale;
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dka + cc * 32 + j),
-                           "f"(__uint_as_float(rk[j]) * a.scale), "f"(__uint_as_float(rk[j + 1]) * a.scale),
-                           "f"(__uint_as_float(rk[j + 2]) * a.scale), "f"(__uint_as_float(rk[j + 3]) * a.scale)
-                           : "memory");
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dva + cc * 32 + j),
-                           "f"(__uint_as_float(rv[j])), "f"(__uint_as_float(rv[j + 1])),
-                           "f"(__uint_as_float(rv[j + 2])), "f"(__uint_as_float(rv[j + 3]))
-                           : "memory");
+          for (int cc = 0; cc < D / 64; ++cc) {
+            uint32_t r[32];
+            tmem_ld_32x32(tm + cc * 32, r);
+            tmem_ld_wait();
+            if (which == 1 && cc + 1 == D / 64) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(acc_drained);
             }
+            if (key_ok) {
+              float4* dst = reinterpret_cast<float4*>(dks + which * plane + cc * 32);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                dst[j] = make_float4(__uint_as_float(r[4 * j]) * f, __uint_as_float(r[4 * j + 1]) * f,
+                                     __uint_as_float(r[4 * j + 2]) * f, __uint_as_float(r[4 * j + 3]) * f);
+            }
+            __syncwarp();
           }
-          __syncwarp();
         }
       }
     }
@@ -1031,11 +1029,11 @@ static int fwd_launch(const ItbAttnArgs* a, int* err, cudaStream_t s) {
 // The passes around the backward kernel: one thread per 8 elements of a [B, T, H D] row, 32-bit index arithmetic
 // while the count allows it.  Both are bound by memory.
 //
-// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d], D / 8 threads per sum; the same threads clear the fp32 accumulators,
-// which were memsets of their own (16 x 1024 x 12 heads of 64: memset, delta and conversion 9.8 + 14.9 + 19.0 us
+// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d], D / 8 threads per sum; the same threads clear the fp32 accumulator of
+// dQ, which was a memset of its own (16 x 1024 x 12 heads of 64: memset, delta and conversion 9.8 + 14.9 + 19.0 us
 // with 64-bit divisions and 4 elements a thread, 15.8 + 10.6 us now).
 template <typename Index>
-__global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D, Index total, Index kv_total) {
+__global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D, Index total) {
   const Index i = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x;
   const int per_head = D >> 3;                                   // threads per sum: 8 or 16
   const Index per_row = static_cast<Index>(a.H) * per_head;
@@ -1052,11 +1050,6 @@ __global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D, Index total, In
     float4* dq = reinterpret_cast<float4*>(a.dq_accum) + static_cast<long long>(i) * 2;
     dq[0] = zero;
     dq[1] = zero;
-    for (Index k = i; k < kv_total; k += total) {
-      float4* dkv = reinterpret_cast<float4*>(a.dkv_accum) + static_cast<long long>(k) * 2;
-      dkv[0] = zero;
-      dkv[1] = zero;
-    }
     const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
     const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y);
 #pragma unroll
@@ -1070,7 +1063,8 @@ __global__ void attn_delta_tc_kernel(const ItbAttnArgs a, int D, Index total, In
   if (mine && c % per_head == 0) a.delta[(static_cast<long long>(b) * a.H + h) * a.T + t] = acc;
 }
 
-// dq (bf16, strided) = the fp32 accumulator; with shared key tiles dk and dv = theirs, [2][B, T, KV, D], too
+// dq (bf16, strided) = the fp32 accumulator; with split key tiles dk and dv = the sums of the shares' slabs
+// [parts][2][B, T, KV, D], those that had a tile, in order
 template <typename Index>
 __global__ void attn_convert_tc_kernel(const ItbAttnArgs a, int D, Index total, Index kv_total) {
   Index i = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x;
@@ -1094,7 +1088,17 @@ __global__ void attn_convert_tc_kernel(const ItbAttnArgs a, int D, Index total, 
   const int c = static_cast<int>(i - r * per_row);
   const int b = static_cast<int>(r / a.T), t = static_cast<int>(r - static_cast<Index>(b) * a.T);
   const float4* v = reinterpret_cast<const float4*>(src) + static_cast<long long>(i) * 2;
-  const float4 lo = v[0], hi = v[1];
+  float4 lo = v[0], hi = v[1];
+  if (src != a.dq_accum) {
+    const int n_qblocks = (a.T + 127) / 128;
+    const int pairs = (n_qblocks - (a.causal ? t / 128 : 0)) * (a.H / a.KV);
+    const long long step = static_cast<long long>(kv_total) * 2;      // float4s of a slab
+    for (int p = 1; p < min(a.bwd_parts, pairs); ++p) {
+      const float4 l = v[p * step], h = v[p * step + 1];
+      lo.x += l.x, lo.y += l.y, lo.z += l.z, lo.w += l.w;
+      hi.x += h.x, hi.y += h.y, hi.z += h.z, hi.w += h.w;
+    }
+  }
   const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
   *reinterpret_cast<uint4*>(dst + b * batch_stride + t * row_stride + c * 8) = pack8(x);
 }
@@ -1130,10 +1134,9 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
   const unsigned delta_blocks = static_cast<unsigned>((vecs + 255) / 256);
   const unsigned convert_blocks = static_cast<unsigned>((vecs + kv_vecs + 255) / 256);
   if (small)
-    attn_delta_tc_kernel<uint32_t><<<delta_blocks, 256, 0, s>>>(*a, D, static_cast<uint32_t>(vecs),
-                                                                static_cast<uint32_t>(kv_vecs));
+    attn_delta_tc_kernel<uint32_t><<<delta_blocks, 256, 0, s>>>(*a, D, static_cast<uint32_t>(vecs));
   else
-    attn_delta_tc_kernel<uint64_t><<<delta_blocks, 256, 0, s>>>(*a, D, vecs, kv_vecs);
+    attn_delta_tc_kernel<uint64_t><<<delta_blocks, 256, 0, s>>>(*a, D, vecs);
   int sms = 0;
   const cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return static_cast<int>(e);
@@ -1154,8 +1157,9 @@ static int bwd_launch(const ItbAttnArgs* a_in, int* err, cudaStream_t s) {
 // CTAs of one (key tile, KV head, batch).  The longest CTA (the first key tile: every query tile of every head of
 // the group) bounds the launch from below, so it is split until it is no longer than an even share of all tiles
 // and a little: one sequence of 2048 tokens with 8 KV heads of 4 query heads has 128 CTAs of up to 64 tiles, 29 a
-// SM.  Each share pays for fp32 accumulators (cleared, added to, converted), so no finer than that.
-// (1 x 2048 tokens, 32 / 8 heads of 64, the whole call: 159 us unsplit, 105 us in two shares.)
+// SM.  Each share pays for fp32 scratch (written, read and converted), so no finer than that.
+// (1 x 2048 tokens, 32 / 8 heads of 64, the whole call: 159 us unsplit, 105 us in two shares; 89 us with the slabs
+// and passes as they are now.)
 extern "C" int itb_flash_attn_bwd_parts(int B, int T, int H, int KV, int causal) {
   if (B <= 0 || T <= 0 || KV <= 0) return 1;
   const long long nt = (T + 127) / 128, G = H / KV;

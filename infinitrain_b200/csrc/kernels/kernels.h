@@ -167,9 +167,8 @@ typedef struct {
   void *dq, *dk, *dv;     // same strides as q, k, v
   float* delta;           // scratch [B, H, T] fp32
   float* dq_accum;        // scratch [B, T, H, D] fp32 (zeroed by the call)
-  // tensor-core backward only, optional: scratch [2][B, T, KV, D] fp32 (zeroed by the call).  When it is
-  // there, the work of a (key tile, KV head, batch) is split into itb_flash_attn_bwd_parts() shares that
-  // sum their dK / dV here.
+  // tensor-core backward only, optional: scratch [parts][2][B, T, KV, D] fp32.  When it is there, the work of
+  // a (key tile, KV head, batch) is split into itb_flash_attn_bwd_parts() shares that put their dK / dV here.
   float* dkv_accum;
   int bwd_parts;          // set by the launcher
 } ItbAttnArgs;
