@@ -182,32 +182,9 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc]; issued by ONE thread.
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with A in TMEM: rows on the lanes, two 16-bit values of consecutive k per 32-bit column
-// (K-major), so a k-step of 16 reads 8 columns.
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same three for a whole, converged warp: one elected thread issues.  With the election inside the
-// instruction's own predicate the loop around it stays warp-uniform, and descriptors and addresses stay in
-// uniform registers; issued from a `lane == 0` branch they are moved there one by one for every MMA.
+// D[tmem] (+)= A[smem desc] * B[smem desc], for a whole, converged warp: one elected thread issues.  With the
+// election inside the instruction's own predicate the loop around it stays warp-uniform, and descriptors and
+// addresses stay in uniform registers; issued from a `lane == 0` branch they are moved there one by one for every MMA.
 __device__ __forceinline__ void umma_f16_ss_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                                   uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -219,6 +196,8 @@ __device__ __forceinline__ void umma_f16_ss_elect(uint32_t tmem_d, uint64_t ades
       : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with A in TMEM: rows on the lanes, two 16-bit values of consecutive k per 32-bit column (K-major), so a
+// k-step of 16 reads 8 columns.
 __device__ __forceinline__ void umma_f16_ts_elect(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
                                                   uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -230,18 +209,13 @@ __device__ __forceinline__ void umma_f16_ts_elect(uint32_t tmem_d, uint32_t tmem
       : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Arrive on an mbarrier once all MMAs issued so far by the warp's elected thread have completed.
 __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
       "elect.sync _|q, 0xffffffff;\n\t"
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar))
       : "memory");
-}
-// Arrive on an mbarrier once all MMAs issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
 }
 // 32 lanes x 32 columns of 32-bit: thread i of the warp receives lane (base+i), columns c..c+31.
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
