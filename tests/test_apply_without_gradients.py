@@ -44,6 +44,26 @@ def test_function_transforms_see_the_autograd_function():
         torch.vmap(lambda t: ops._apply(_Twice, t))(torch.ones(2, 3))
 
 
+class _FilledElsewhere(torch.autograd.Function):
+    """2 x + 1, written by something the tracer does not see, as a kernel launch is."""
+
+    @staticmethod
+    def forward(ctx, x):
+        out = torch.empty_like(x)
+        out.numpy()[...] = 2 * x.numpy() + 1
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        return 2 * dy
+
+
+def test_a_trace_without_gradients_runs_the_function_again():
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda x: ops._apply(_FilledElsewhere, x), torch.ones(3), check_trace=False)
+        assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 11.0))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("family", ["gpt2", "llama3"])
 def test_logits_are_the_same_with_and_without_gradients(family):
