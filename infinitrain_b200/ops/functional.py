@@ -66,9 +66,9 @@ def _apply(fn, *args):
     is nothing for autograd to record or refuse, and the forward is called as it is: ``apply`` costs the host about
     10 us an op, as much as the launch (12 layers of width 768 on 1 x 96 tokens, bound by the host: 2.94 -> 2.22 ms).
     A tracer records the applied function as a node that runs again; of a bare forward it would see the allocation of
-    the output and nothing of the launch that fills it."""
+    the output and nothing of the launch that fills it.  A profiler takes the op's name from ``apply``."""
     if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
-            or torch._C._get_tracing_state() is not None):
+            or torch._C._get_tracing_state() is not None or torch._C._autograd._profiler_enabled()):
         return fn.apply(*args)
     return fn.forward(_NoContext(), *args)
 

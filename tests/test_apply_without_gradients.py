@@ -64,6 +64,12 @@ def test_a_trace_without_gradients_runs_the_function_again():
         assert torch.equal(traced(torch.full((3,), 5.0)), torch.full((3,), 11.0))
 
 
+def test_a_profile_without_gradients_names_the_op():
+    with torch.no_grad(), torch.autograd.profiler.profile() as prof:
+        ops._apply(_Twice, torch.ones(3))
+    assert "_Twice" in [event.name for event in prof.function_events]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("family", ["gpt2", "llama3"])
 def test_logits_are_the_same_with_and_without_gradients(family):
