@@ -591,9 +591,10 @@ def swiglu_packed(ab):
 
 
 def _rows_for_kernel(x: torch.Tensor) -> torch.Tensor:
-    """``x`` as rows that the kernels can read in 16-byte pieces; a copy only when it is not laid out so."""
+    """``x`` as rows that the kernels can read in 16-byte pieces, a multiple of 8 elements apart (4 fp32 would be
+    aligned too, but the kernels refuse it); a copy only when it is not laid out so."""
     x2 = x.reshape(-1, x.shape[-1])
-    if x2.stride(-1) != 1 or x2.stride(0) * x2.element_size() % 16 or x2.data_ptr() % 16:
+    if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
         x2 = x2.clone(memory_format=torch.contiguous_format)
     return x2
 

@@ -3,19 +3,34 @@ bits, whatever the layout of the inputs and of the gradient."""
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rows_for_kernel_are_laid_out_as_the_kernels_want_them(dtype):
+    from infinitrain_b200.ops import functional as ops
+
+    for width in (8, 12, 16, 20, 24):
+        base = torch.randn(5, width).to(dtype)
+        for rows in (base, base[:1], base[2:3]):
+            for first in range(width - 7):
+                x = rows[:, first:first + 8]
+                y = ops._rows_for_kernel(x)
+                assert torch.equal(x, y)
+                assert y.stride(1) == 1 and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0
 
 
 def _layouts(rows, F, dtype):
     wide = torch.randn(rows, 2 * F + 24, device="cuda").to(dtype)
     yield torch.randn(rows, F, device="cuda").to(dtype), torch.randn(rows, F, device="cuda").to(dtype)
     yield wide[:, :F], wide[:, F:2 * F]                    # rows of one wider matrix
+    narrow = torch.randn(rows, F + 4, device="cuda").to(dtype)
+    yield narrow[:, :F], narrow[:, 4:]                     # rows a multiple of 4, not of 8 elements apart
     yield wide[:, 8:F + 8], torch.randn(rows, F, device="cuda").to(dtype)     # unequal row strides
     yield wide[:, 1:F + 1], wide[:, F + 3:2 * F + 3]       # off the 16-byte boundary
     yield torch.randn(F, rows, device="cuda").to(dtype).t(), wide[:, :F]      # columns contiguous
     yield wide[:1, :F].expand(rows, F), wide[:, :F]        # one row for all
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,F", [(1, 8), (7, 264), (300, 1032)])
 def test_swiglu_pair_is_swiglu(rows, F, dtype):
