@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <initializer_list>
 
 #include "kernels.h"
 
@@ -365,10 +366,18 @@ extern "C" int itb_gelu_bwd(const void* dy, const void* x, void* dx, int dtype, 
   return static_cast<int>(cudaGetLastError());
 }
 
+// The SwiGLU kernels read and write pieces of 16 bytes.
+static bool aligned16(std::initializer_list<const void*> pointers) {
+  for (const void* p : pointers)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
 extern "C" int itb_swiglu_fwd(const void* a, const void* b, long long ld_in, void* out,
                               long long ld_out, int dtype, int rows, int F, cudaStream_t s) {
   if (rows <= 0 || F <= 0) return 0;
   if (F % 8 || ld_in % 8 || ld_out % 8) return -3;
+  if (!aligned16({a, b, out})) return -2;
   const long long work = static_cast<long long>(rows) * (F / 8);
   if (dtype == kItbBF16)
     swiglu_fwd_kernel<__nv_bfloat16><<<pw_grid(work), kPwThreads, 0, s>>>(
@@ -385,6 +394,7 @@ extern "C" int itb_swiglu_bwd(const void* dout, long long ld_dout, const void* a
                               int rows, int F, cudaStream_t s) {
   if (rows <= 0 || F <= 0) return 0;
   if (F % 8 || ld_in % 8 || ld_dout % 8 || ld_dab % 8) return -3;
+  if (!aligned16({dout, a, b, da, db})) return -2;
   const long long work = static_cast<long long>(rows) * (F / 8);
   if (dtype == kItbBF16)
     swiglu_bwd_kernel<__nv_bfloat16><<<pw_grid(work), kPwThreads, 0, s>>>(

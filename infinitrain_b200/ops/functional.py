@@ -555,6 +555,15 @@ def gelu(x):
     return ref.new_gelu(x)
 
 
+def _rows_for_kernel(x: torch.Tensor) -> torch.Tensor:
+    """``x`` as rows that the kernels can read in 16-byte pieces, a multiple of 8 elements apart (4 fp32 would be
+    aligned too, but the kernels refuse it); a copy only when it is not laid out so."""
+    x2 = x.reshape(-1, x.shape[-1])
+    if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+        x2 = x2.clone(memory_format=torch.contiguous_format)
+    return x2
+
+
 class _SwiGLUFn(torch.autograd.Function):
     """out = a * silu(b) for a, b the two column halves of one [rows, 2F] matrix."""
 
@@ -562,8 +571,7 @@ class _SwiGLUFn(torch.autograd.Function):
     def forward(ctx, ab):
         C = _C()
         F = ab.shape[-1] // 2
-        ab2 = ab.reshape(-1, 2 * F)
-        ab2 = ab2 if ab2.stride(-1) == 1 else ab2.contiguous()
+        ab2 = _rows_for_kernel(ab)
         out = C.swiglu_fwd(ab2[:, :F], ab2[:, F:])
         _counters["launches"] += 1
         ctx.save_for_backward(ab2)
@@ -575,9 +583,7 @@ class _SwiGLUFn(torch.autograd.Function):
         C = _C()
         (ab2,) = ctx.saved_tensors
         F = ab2.shape[-1] // 2
-        d2 = dout.reshape(-1, F).to(ab2.dtype)
-        d2 = d2 if d2.stride(-1) == 1 else d2.contiguous()
-        dab = C.swiglu_bwd(d2, ab2[:, :F], ab2[:, F:])
+        dab = C.swiglu_bwd(_rows_for_kernel(dout.to(ab2.dtype)), ab2[:, :F], ab2[:, F:])
         _counters["launches"] += 1
         return dab.view(ctx.shape)
 
@@ -588,15 +594,6 @@ def swiglu_packed(ab):
     if ab.is_cuda and ab.dtype in (torch.float32, torch.bfloat16) and F % 8 == 0 and _ext.available():
         return _apply(_SwiGLUFn, ab)
     return ref.swiglu(ab[..., :F], ab[..., F:])
-
-
-def _rows_for_kernel(x: torch.Tensor) -> torch.Tensor:
-    """``x`` as rows that the kernels can read in 16-byte pieces, a multiple of 8 elements apart (4 fp32 would be
-    aligned too, but the kernels refuse it); a copy only when it is not laid out so."""
-    x2 = x.reshape(-1, x.shape[-1])
-    if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
-        x2 = x2.clone(memory_format=torch.contiguous_format)
-    return x2
 
 
 class _SwiGLUPairFn(torch.autograd.Function):

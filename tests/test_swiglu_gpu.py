@@ -44,7 +44,55 @@ def test_swiglu_pair_is_swiglu(rows, F, dtype):
             for fn in (ops.swiglu_pair, ops.swiglu):
                 x, y = a.detach().requires_grad_(), b.detach().requires_grad_()
                 out = fn(x, y)
-                # swiglu wants an aligned gradient (contiguous() leaves a single row where it is)
-                g = dout.clone(memory_format=torch.contiguous_format) if fn is ops.swiglu else dout
-                results.append((out, *torch.autograd.grad(out, (x, y), g)))
+                results.append((out, *torch.autograd.grad(out, (x, y), dout)))
             assert all(torch.equal(p, q) for p, q in zip(*results))
+
+
+class _AlignedOnly:
+    """The extension's two entries with what their kernels want of a layout, on the CPU."""
+
+    @staticmethod
+    def _check(*tensors):
+        for t in tensors:
+            assert t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+    def swiglu_fwd(self, a, b):
+        self._check(a, b)
+        return a * torch.nn.functional.silu(b)
+
+    def swiglu_bwd(self, dout, a, b):
+        self._check(dout, a, b)
+        s = torch.sigmoid(b)
+        return torch.cat([dout * b * s, dout * a * (s + b * s * (1 - s))], dim=1)
+
+
+def test_swiglu_of_a_copy_hands_the_kernels_aligned_rows(monkeypatch):
+    from infinitrain_b200.ops import functional as ops
+
+    monkeypatch.setattr(ops, "_C", lambda: _AlignedOnly())
+    F = 8
+    for rows in (1, 3):
+        wide = torch.randn(rows, 2 * F + 8)
+        for ab in (wide[:, :2 * F], wide[:, 1:2 * F + 1], torch.randn(rows, 2 * F + 4)[:, 4:], torch.randn(2 * F, rows).t()):
+            ab = ab.detach().requires_grad_()
+            out = ops._SwiGLUFn.apply(ab)
+            dout = torch.randn(rows, F + 8)[:, 3:F + 3]
+            (got,) = torch.autograd.grad(out, ab, dout)
+            a, b = ab.detach()[:, :F].requires_grad_(), ab.detach()[:, F:].requires_grad_()
+            ref = a * torch.nn.functional.silu(b)
+            assert torch.allclose(out, ref)
+            assert torch.allclose(got, torch.cat(torch.autograd.grad(ref, (a, b), dout), dim=1), atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_swiglu_kernels_refuse_what_is_off_the_boundary(dtype):
+    from infinitrain_b200 import _ext
+
+    C = _ext.load(required=True)
+    good, wide = torch.randn(4, 16, device="cuda").to(dtype), torch.randn(4, 24, device="cuda").to(dtype)
+    off = wide[:, 1:17]         # the host looks at the pointer: nothing is launched
+    with pytest.raises(RuntimeError):
+        C.swiglu_fwd(off, off)
+    with pytest.raises(RuntimeError):
+        C.swiglu_bwd(off, good, good)
