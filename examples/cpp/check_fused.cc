@@ -62,6 +62,9 @@ int main() {
   both([](auto& v) { return itb::ops::rmsnorm(v[0], v[1], 1e-5); }, {x, g1}, "rmsnorm");
   both([](auto& v) { return itb::ops::gelu(v[0]); }, {x}, "gelu");
   both([](auto& v) { return itb::ops::swiglu(v[0], v[1]); }, {x, x * 0.7 + 0.1}, "swiglu");
+  // the gradient that swiglu gets is a column range that begins off the 16-byte boundary, in rows 8 elements longer
+  both([](auto& v) { return torch::cat({v[0].narrow(-1, 0, 1), itb::ops::swiglu(v[0], v[1]), v[0].narrow(-1, 0, 7)}, -1); },
+       {x, x * 0.7 + 0.1}, "swiglu, gradient off boundary");
   for (int64_t D : {64, 128}) {
     const int64_t B = 2, T = 256, H = 4, KV = 2;
     Tensor qkv = torch::randn({B, T, (H + 2 * KV) * D}) * 0.5;

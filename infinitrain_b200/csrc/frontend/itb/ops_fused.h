@@ -94,6 +94,14 @@ inline Tensor as_bf16_2d(const Tensor& x) {
   return x2;
 }
 
+// x as rows that the SwiGLU kernels can read in 16-byte pieces; a copy only when it is not laid out so.
+inline Tensor rows_for_kernel(const Tensor& x) {
+  Tensor x2 = x.reshape({-1, x.size(-1)});
+  if (x2.stride(-1) != 1 || x2.stride(0) % 8 || reinterpret_cast<uintptr_t>(x2.data_ptr()) % 16)
+    x2 = x2.clone(at::MemoryFormat::Contiguous);
+  return x2;
+}
+
 // C[M, N] (+)= A . B with the layout flags of kernels.h, on CTA pairs.
 inline void gemm(const Tensor& a, bool a_mn, const Tensor& b, bool b_mn, int64_t M, int64_t N, int64_t K, Tensor& c,
                  const Tensor& c2, const Tensor& bias, const Tensor& residual, const Tensor& aux, int flags) {
@@ -293,8 +301,7 @@ inline Tensor gelu(const Tensor& x) { return GeluFn::apply(x); }
 struct SwiGLUFn : public torch::autograd::Function<SwiGLUFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& ab) {
     int64_t F = ab.size(-1) / 2;
-    Tensor ab2 = ab.reshape({-1, 2 * F});
-    if (ab2.stride(-1) != 1) ab2 = ab2.contiguous();
+    Tensor ab2 = rows_for_kernel(ab);
     int64_t rows = ab2.size(0), eb = ab2.element_size();
     Tensor out = torch::empty({rows, F}, ab2.options().requires_grad(false));
     const char* base = static_cast<const char*>(ab2.data_ptr());
@@ -310,9 +317,8 @@ struct SwiGLUFn : public torch::autograd::Function<SwiGLUFn> {
     ITB_PROFILE("swiglu[bwd]", grads[0]);
     Tensor ab2 = ctx->get_saved_variables()[0];
     int64_t F = ab2.size(1) / 2, rows = ab2.size(0), eb = ab2.element_size();
-    Tensor d2 = grads[0].reshape({-1, F}).to(ab2.scalar_type());
-    if (d2.stride(-1) != 1) d2 = d2.contiguous();
-    Tensor dab = torch::empty_like(ab2);
+    Tensor d2 = rows_for_kernel(grads[0].to(ab2.scalar_type()));
+    Tensor dab = torch::empty({rows, 2 * F}, ab2.options());
     const char* base = static_cast<const char*>(ab2.data_ptr());
     char* dbase = static_cast<char*>(dab.data_ptr());
     check(itb_swiglu_bwd(d2.data_ptr(), d2.stride(0), base, base + F * eb, ab2.stride(0), dbase, dbase + F * eb,
