@@ -29,16 +29,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred = 0;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "elect.sync _|P, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(pred));
-  return pred != 0;
-}
-
 // A warpgroup (four warps, all of them) takes registers from or gives them back to what its CTA was launched with.
 template <int N>
 __device__ __forceinline__ void regs_grow() {
@@ -342,14 +332,6 @@ __device__ __forceinline__ void umma_f16_ss_pair_elect(uint32_t tmem_d, uint64_t
       : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive (once the MMAs issued so far have completed) on ONE mbarrier given by its shared::cluster
-// address: the leader signals its own barrier and, with a second commit, the peer's.
-__device__ __forceinline__ void umma_commit_pair(uint32_t mbar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   mbar_cluster_addr)
-               : "memory");
-}
-
 // One commit that arrives on the mbarrier at the same shared-memory offset in every CTA of `cta_mask`
 // (the pair: 0b11).  Signals only: no data moves, this is not a load.
 // For a whole, converged warp: one elected thread issues.
