@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module", params=["pair", "single"])
 def C(request):
-    """Every kernel test runs with both GEMM kernels: CTA pairs (cta_group::2) and single CTAs."""
+    """Every kernel test runs with both GEMM kernels: CTA pairs (cta_group::2) and single CTAs.  Outputs of at most
+    one wave of 128 x 64 tiles have a kernel of their own in either mode; the GEMM tests have sizes above that too."""
     from infinitrain_b200 import _ext
 
     mod = _ext.load(required=True)
@@ -25,7 +26,7 @@ def _rel(a, b):
 
 
 GEMM_SHAPES = [(128, 256, 64), (256, 512, 128), (200, 264, 72), (1024, 768, 768), (384, 2304, 768),
-               (130, 50264, 64)]
+               (130, 50264, 64), (1153, 1032, 264), (2331, 768, 128)]
 
 
 @pytest.mark.parametrize("M,N,K", GEMM_SHAPES)
@@ -39,7 +40,8 @@ def test_gemm_forward_layout(C, M, N, K):
     assert _rel(c, ref) < 1e-2
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 512, 128), (200, 264, 72), (1024, 768, 3072)])
+@pytest.mark.parametrize("M,N,K", [(256, 512, 128), (200, 264, 72), (1024, 768, 3072), (1153, 1032, 264),
+                                   (2331, 768, 1024)])
 def test_gemm_dgrad_layout(C, M, N, K):
     # dx[M,K'] = dy[M,N'] @ W[N',K'] : A K-major (contraction N'), B MN-major.
     torch.manual_seed(1)
@@ -66,9 +68,9 @@ def test_gemm_wgrad_layout_splitk(C, M, N, K):
     assert _rel(c2, ref) < 1e-3
 
 
-def test_gemm_epilogues(C):
+@pytest.mark.parametrize("M,N,K", [(512, 768, 256), (1153, 1032, 256), (2331, 768, 256)])
+def test_gemm_epilogues(C, M, N, K):
     torch.manual_seed(3)
-    M, N, K = 512, 768, 256
     a = torch.randn(M, K, device="cuda").bfloat16()
     b = (torch.randn(N, K, device="cuda") / math.sqrt(K)).bfloat16()
     bias = torch.randn(N, device="cuda")
