@@ -118,6 +118,9 @@ def _as_bf16_2d(x: torch.Tensor) -> torch.Tensor:
         x2 = x2.to(torch.bfloat16)
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
         x2 = x2.contiguous()
+    if x2.stride(0) % 8:        # TMA wants rows a multiple of 16 bytes apart; the gradient of a rank-4 product's are not
+        padded = x2.new_empty(x2.shape[0], (x2.shape[1] + 7) // 8 * 8)
+        x2 = padded[:, :x2.shape[1]].copy_(x2)
     return x2
 
 
@@ -182,17 +185,13 @@ class _LinearFn(torch.autograd.Function):
         d_res = dy if ctx.has_res else None
         if d_res is not None and d_res.dtype != ctx.res_dtype:
             d_res = d_res.to(ctx.res_dtype)
-        dy2 = dy.reshape(M, N)
-        if dy2.dtype != torch.bfloat16:
-            dy2 = dy2.to(torch.bfloat16)
-        if dy2.stride(-1) != 1 or (dy2.stride(0) % 8) or (dy2.data_ptr() % 16):
-            dy2 = dy2.contiguous()
+        dy2 = _as_bf16_2d(dy)
         if ctx.gelu:
             # dy is the gradient of the activation output: fold gelu'(h) in with one pointwise pass.
             dyc = dy2 if dy2.is_contiguous() else dy2.contiguous()
             prec = pre[:, :N] if ctx.ld != N else pre
             prec = prec if prec.is_contiguous() else prec.contiguous()
-            dy2 = C.gelu_bwd(dyc, prec)
+            dy2 = _as_bf16_2d(C.gelu_bwd(dyc, prec))
             _counters["launches"] += 1
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
