@@ -644,10 +644,15 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 //   online softmax: one thread per query row holds its row of S in registers, so nothing crosses threads;
 //   P goes as bf16 over the spent S in TMEM
 //   O[m,d] += P[m,n] V[n,d]      tcgen05.mma  P (from TMEM) x V (MN-major)       -> TMEM, D columns a tile
-// While four warps do the softmax of one tile, the tensor core works on the other.  O stays in TMEM: it is
-// multiplied by exp2(m_old - m_new) only when a row's maximum has grown by more than kGrowth since the last time,
-// until then P is taken relative to the older maximum (at most 2^kGrowth large; the final division is exact either
-// way).  Persistent, one CTA per SM; the next item's loads and first S run under the last steps of the one before.
+// While four warps do the softmax of one tile, the tensor core works on the other.  O stays in TMEM: a warp reads it,
+// multiplies it by exp2(m_old - m_new) and writes it back when the maximum of one of its rows has grown, after its P
+// of the step.  (Left relative to an older maximum until that is 2^8 behind, O is rescaled once or twice a row, but the
+// largest probabilities are then no longer 1 and are rounded to bf16 like the others: 1 to 2 % more error against 64
+// bits, for nothing at head size 64 and 459 -> 417 us of the 8192-token case below.)  Persistent, one CTA per SM; the
+// next item's loads and first S run under the last steps of the one before.
+//
+// Two query tiles in turn, warp roles and P as the MMA's operand in TMEM are published techniques of flash attention
+// for this architecture (FlashAttention-4).
 //
 // What bounds it: the exponentials, 16 per cycle and SM: 1024 cycles per 128 x 128 scores (head size 128: the two
 // contractions take as long).
@@ -668,7 +673,6 @@ struct FwdCfg {
   static_assert(kSmem <= 232448, "shared memory of one SM");
 };
 constexpr int kFwdThreads = 320;     // 2 x 4 softmax warps, TMA warp, MMA warp
-constexpr float kGrowth = 8.f;
 
 struct FwdItems {
   int pairs, HB, H, causal, n_blocks, T;
@@ -881,8 +885,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     while (ok && item.next()) {
       const int steps = t ? item.steps[1] : item.steps[0], mb = item.m0 / 128 + t;
       if (steps == 0) continue;
-      float base = 0.f;                 // what the exponents are relative to (scaled, log2 domain)
-      float l_run = 0.f;
+      float m_run = -INFINITY, l_run = 0.f;      // running maximum (scaled, log2 domain) and sum
       for (int j = 0; j < steps; ++j, ++n) {
         ok = wait(&s_full[t], n);
         if (!ok) break;
@@ -902,29 +905,15 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < 128; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(s[i >> 5][i & 31]));
-        // sl2 > 0: scaling commutes with the maximum.  A row that has seen no key yet (l_run = 0) takes any finite
-        // maximum as its base, and 0 for none, so that exp2 yields 0, not NaN.
+        // sl2 > 0: scaling commutes with the maximum.  A row that has seen no key yet takes 0 as its base, so that exp2
+        // yields 0, not NaN.
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
-        const bool fresh = l_run == 0.f;
-        if (j == 0) {
-          base = mx == -INFINITY ? 0.f : mx;
-        } else if (__any_sync(~0u, fresh || mx > base + kGrowth)) {
-          const float new_base = fresh ? (mx == -INFINITY ? 0.f : mx) : fmaxf(base, mx);
-          const float corr = fresh ? 0.f : ex2(base - new_base);
-          l_run *= corr;
-          base = new_base;
-          // s_full says that the PV of the step before has completed
-#pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x16(tO + c * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-            tmem_st_32x16(tO + c * 16, o);
-          }
-        }
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        const float m_new = fmaxf(m_run, mx);
+        const float base = m_new == -INFINITY ? 0.f : m_new;
+        const float corr = ex2(m_run - base);
+        const bool rescale = j > 0 && __any_sync(~0u, m_new > m_run);
+        m_run = m_new;
+        float sum = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t w[16];
@@ -932,13 +921,27 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           for (int i = 0; i < 16; ++i) {
             const float p0 = ex2(fmaf(__uint_as_float(s[c][2 * i]), sl2, -base));
             const float p1 = ex2(fmaf(__uint_as_float(s[c][2 * i + 1]), sl2, -base));
-            sum[(2 * i) & 3] += p0;
-            sum[(2 * i + 1) & 3] += p1;
+            sum += p0;
+            sum += p1;
             w[i] = pack2(p0, p1);
           }
           tmem_st_32x16(tS + c * 16, w);
         }
-        l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        l_run = l_run * corr + sum;
+        // s_full says that the PV of the step before has completed; S is spent, its registers take O on its way through
+        if (rescale) {
+          uint32_t o[D / 32][32];
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) tmem_ld_32x32(tO + c * 32, o[c]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(__uint_as_float(o[c >> 1][(c & 1) * 16 + i]) * corr);
+            tmem_st_32x16(tO + c * 16, w);
+          }
+        }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
@@ -979,7 +982,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
       if (qrow < a.T)
         a.lse[(static_cast<long long>(item.b) * a.H + item.h) * a.T + qrow] =
-            l_run > 0.f ? base * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
+            l_run > 0.f ? m_run * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
       __syncwarp();
     }
     if (!ok) give_up(215);
