@@ -879,7 +879,9 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tm_S + t * 128 + lane_addr, tO = tm_O + t * D + lane_addr;
-    const float sl2 = a.scale * kLog2e;
+    // a masked key's score is the infinity whose probability is 0; no score times a scale of 0 is that
+    const float sl2 = a.scale == 0.f ? FLT_MIN : a.scale * kLog2e;
+    const float hidden = sl2 > 0.f ? -INFINITY : INFINITY;
     bool ok = true;
     uint32_t n = 0, items = 0;
     while (ok && item.next()) {
@@ -900,13 +902,13 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
           const int n_lim = min(diag ? row + 1 : 128, a.T - j * 128);   // keys [0, n_lim) visible
 #pragma unroll
           for (int i = 0; i < 128; ++i)
-            if (i >= n_lim) s[i >> 5][i & 31] = __float_as_uint(-INFINITY);
+            if (i >= n_lim) s[i >> 5][i & 31] = __float_as_uint(hidden);
         }
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < 128; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(s[i >> 5][i & 31]));
-        // sl2 > 0: scaling commutes with the maximum.  A row that has seen no key yet takes 0 as its base, so that exp2
-        // yields 0, not NaN.
+        // sl2 > 0: scaling commutes with the maximum (below 0 the lowest score, or none, serves as well).  A row without a
+        // maximum takes 0 as its base, so that exp2 yields 0, not NaN.
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
         const float m_new = fmaxf(m_run, mx);
         const float base = m_new == -INFINITY ? 0.f : m_new;
@@ -982,7 +984,7 @@ flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
       if (qrow < a.T)
         a.lse[(static_cast<long long>(item.b) * a.H + item.h) * a.T + qrow] =
-            l_run > 0.f ? m_run * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
+            l_run > 0.f ? (m_run == -INFINITY ? 0.f : m_run) * 0.6931471805599453f + logf(l_run) : -FLT_MAX;
       __syncwarp();
     }
     if (!ok) give_up(215);

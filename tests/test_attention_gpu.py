@@ -102,3 +102,19 @@ def test_probabilities_are_relative_to_the_maximum_so_far():
     # half a unit in the last place of bf16, and what fp32 leaves: exponents to 2^-21, exp2 and the sum to 2^-22
     unit = torch.ldexp(torch.ones_like(ref), torch.frexp(ref).exponent - 8)
     assert ((o.double() - ref).abs() <= 0.5 * unit + 2.0 ** -19 * ref.abs() + 1e-9).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+def test_masked_keys_stay_hidden_whatever_the_scale(D, scale):
+    from infinitrain_b200 import _ext
+
+    C = _ext.load(required=True)
+    torch.manual_seed(D)
+    q, k, v = torch.randn(3, 2, 300, 2, D, device="cuda").bfloat16()
+    for causal in (True, False):                            # the diagonal tile, the ragged last one
+        o, lse = C.flash_attn_fwd(q, k, v, scale, causal)
+        ref, ref_lse = _attend(q, k, v, scale, causal)
+        assert C.kernel_status() == 0
+        assert (lse.double() - ref_lse).abs().max() < 1e-4
+        assert ((o.double() - ref).norm(dim=-1) / ref.norm(dim=-1)).max() < TOLERANCE
