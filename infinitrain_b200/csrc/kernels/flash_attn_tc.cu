@@ -1170,7 +1170,9 @@ extern "C" int itb_flash_attn_bwd_parts(int B, int T, int H, int KV, int causal)
   const long long nt = (T + 127) / 128, G = H / KV;
   const long long most = nt * G;                             // tiles of the longest CTA
   const long long tiles = (causal ? nt * (nt + 1) / 2 : nt * nt) * G * KV * B;
-  const long long share = tiles / 148 + tiles / (148 * 8) + 1;
+  int sms = 0;
+  if (itb::fatc::sm_count(&sms) != cudaSuccess || sms <= 0) sms = 148;     // of a B200, where there is no device to ask
+  const long long share = tiles / sms + tiles / (sms * 8) + 1;
   int parts = 1;
   while (parts < 16 && parts < most && (most + parts - 1) / parts > share) ++parts;
   return parts;
