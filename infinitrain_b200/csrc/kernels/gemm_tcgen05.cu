@@ -15,8 +15,8 @@
 //   wgrad     dW = dy^T x       A = dy [M,N] MN-major, B = x [M,K] MN-major (contraction M)
 //
 // Kernel shape: persistent, one CTA per SM, 192 threads = 1 TMA warp + 1 MMA warp + 4 epilogue
-// warps; tile 128 x BN x 64 with a 4-deep shared-memory ring and two TMEM accumulators so that
-// the epilogue of tile i overlaps the main loop of tile i+1.
+// warps; tile 128 x BN x 64 with a ring of 4 stages in shared memory (BN 256) or 8 (BN 64) and two TMEM
+// accumulators so that the epilogue of tile i overlaps the main loop of tile i+1.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>

@@ -52,7 +52,7 @@ typedef struct {
 int itb_gemm_bf16(const ItbGemmArgs* args, cudaStream_t stream);
 // Whether the output is small enough for itb_gemm_bf16's 128 x 64 tiles to run all at once (no accumulation).
 int itb_gemm_narrow(const ItbGemmArgs* args);
-// Same contract, computed by CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair).
+// Same contract, computed by CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair) unless the output is that small.
 int itb_gemm_bf16_pair(const ItbGemmArgs* args, cudaStream_t stream);
 
 // ------------------------------------------------------------------ normalisation
