@@ -23,7 +23,7 @@
 // What bounds it: the exponentials (16 per cycle and SM: 1024 cycles a tile) and the five contractions (1280
 // cycles a tile at head size 64, 2560 at 128).
 // Measured (this kernel alone, causal): 16 x 1024 tokens, 12 heads of 64: 280 us when one warp set walked the whole
-// chain of a tile, one CTA per key tile; 147 us now.  1 x 8192, 32 query and 8 KV heads of 128: 3018 -> 1400 us.
+// chain of a tile, one CTA per key tile; 147 us now.  1 x 8192, 32 query and 8 KV heads of 128: 3018 -> 1435 us.
 // 1 x 2048, 32 / 8 heads of 64: 292 -> 75 us.  A tile takes 3260 cycles at head size 64 and 5000 at 128, where shared
 // memory is busy most of the time: 288 KB of operands, 128 KB for dQ's way out and 96 KB of loads and dS a tile at
 // 128 bytes a cycle are 4100 cycles.
@@ -648,7 +648,7 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 // multiplies it by exp2(m_old - m_new) and writes it back when the maximum of one of its rows has grown, after its P
 // of the step.  (Left relative to an older maximum until that is 2^8 behind, O is rescaled once or twice a row, but the
 // largest probabilities are then no longer 1 and are rounded to bf16 like the others: 1 to 2 % more error against 64
-// bits, for nothing at head size 64 and 459 -> 417 us of the 8192-token case below.)  Persistent, one CTA per SM; the
+// bits, for nothing at head size 64 and 476 -> 437 us of the 8192-token case below.)  Persistent, one CTA per SM; the
 // next item's loads and first S run under the last steps of the one before.
 //
 // Two query tiles in turn, warp roles and P as the MMA's operand in TMEM are published techniques of flash attention
@@ -657,7 +657,7 @@ flash_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 // What bounds it: the exponentials, 16 per cycle and SM: 1024 cycles per 128 x 128 scores (head size 128: the two
 // contractions take as long).
 // Measured (causal): 16 x 1024 tokens, 12 heads of 64: 109 us with one tile per CTA, P through shared memory and O
-// added up in registers; 66 us now.  1 x 8192, 32 / 8 heads of 128: 1243 -> 437 us (1258 TFLOP/s, 0.77 of the
+// added up in registers; 66 us now.  1 x 8192, 32 / 8 heads of 128: 1243 -> 476 us (1155 TFLOP/s, 0.70 of the
 // measured GEMM peak).  1 x 2048, 32 / 8 heads of 64: 80 -> 35 us.
 template <int D>
 struct FwdCfg {

@@ -406,8 +406,11 @@ extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
   // 128 x 64 tiles where they all run at once: a small output has too few 256-wide tiles to fill the machine (96 x 768
   // has three), and each walks over the whole contraction by itself.
   // 96 x 768 x 3072: 28.7 -> 19.5 us, 256 x 3072 x 768 (one CTA pair per 256 x 256 before): 16.4 -> 12.3 us, the
-  // forward and input-gradient GEMMs of GPT-2 124M on 4 x 64 tokens: 2.11 -> 1.38 ms.  Above the line both forms
-  // need more than one wave and the pairs read their operands half as often.
+  // forward and input-gradient GEMMs of GPT-2 124M on 4 x 64 tokens: 2.11 -> 1.38 ms.
+  // The line lies where these tiles need a second wave, which pairs need only from 75 tiles of 256 x 256 on.  Pairs
+  // against these tiles, us with the operands not in L2: 1152 x 1024 (144 tiles) at K 768 / 3072 / 8192 15.9 / 27.2 / 50.2
+  // against 12.3 / 20.5 / 39.0; 1153 x 1024 (160 tiles) 15.3 / 27.5 / 50.2 against 14.4 / 31.2 / 67.5; 2304 x 1024 (288)
+  // 16.5 / 28.7 / 54.1 against 15.2 / 32.7 / 69.6; 4096 x 1024 (512) 17.4 / 29.7 / 57.3 against 22.5 / 57.2 / 131.2.
   const bool narrow = itb_gemm_narrow(a);
   const int BN = narrow ? 64 : 256;
   if (!a->b_mn_major)

@@ -166,8 +166,9 @@ def bench_attention(C):
 
 
 def profile_case(C):
-    """GEMM forward (twice) and weight gradient on 16384 x 2304 x 768, attention forward and backward on
-    16 x 1024 x 12 heads x 64: the launches a profiler capture of the top kernels needs, and no more."""
+    """GEMM forward (twice) and weight gradient on 16384 x 2304 x 768, a GEMM of a small output (96 x 768 x 3072),
+    attention forward and backward on 16 x 1024 x 12 heads x 64: the launches a profiler capture of the top kernels
+    needs, and no more."""
     M, N, K = 16384, 2304, 768
     a = torch.randn(M, K, device="cuda").bfloat16()
     b = torch.randn(N, K, device="cuda").bfloat16()
@@ -176,6 +177,9 @@ def profile_case(C):
         C.gemm(a, False, b, False, M, N, K, c, None, None, None, None, 0, 0)
     dw = torch.zeros(N, K, device="cuda")
     C.gemm(c, True, a, True, N, K, M, dw, None, None, None, None, C.GEMM_OUT_F32 | C.GEMM_ATOMIC, 0)
+    a, b = torch.randn(96, 3072, device="cuda").bfloat16(), torch.randn(768, 3072, device="cuda").bfloat16()
+    C.gemm(a, False, b, False, 96, 768, 3072, torch.empty(96, 768, device="cuda", dtype=torch.bfloat16), None, None, None,
+           None, 0, 0)
     q, k, v, dq, dk, dv = _attn_tensors(16, 1024, 12, 12, 64)
     o, lse = C.flash_attn_fwd(q, k, v, 0.125, True)
     C.flash_attn_bwd(torch.randn_like(o), q, k, v, o, lse, dq, dk, dv, 0.125, True)
