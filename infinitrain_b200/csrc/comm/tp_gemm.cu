@@ -38,14 +38,14 @@ namespace pair {
 template <bool A_MN, bool B_MN>
 static int launch_tp(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tc2,
                      const CUtensorMap& te, const GemmDev& p, const TpDev& tp, int pairs, cudaStream_t stream) {
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, true>;
-  constexpr int smem = kSmemTotal + 1024;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, true, false>;
+  constexpr int smem = Cfg<true, false>::kSmemLaunch;
   static PerDeviceOnce configured;
   if (configured.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  kern<<<2 * pairs, kThreads, smem, stream>>>(ta, tb, tc, tc2, te, p, tp);
+  kern<<<2 * pairs, Cfg<true, false>::kThreads, smem, stream>>>(ta, tb, tc, tc2, te, p, tp);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "gemm_pair_body.cuh"
 
@@ -29,17 +30,17 @@ int make_tmap_f32_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t
 
 namespace pair {
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool kWide>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tc2,
                   const CUtensorMap& te, const GemmDev& p, int pairs, cudaStream_t stream) {
-  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, false>;
-  constexpr int smem = kSmemTotal + 1024;
+  auto kern = gemm_bf16_pair_kernel<A_MN, B_MN, false, kWide>;
+  constexpr int smem = Cfg<false, kWide>::kSmemLaunch;
   static PerDeviceOnce configured;
   if (configured.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  kern<<<2 * pairs, kThreads, smem, stream>>>(ta, tb, tc, tc2, te, p, TpDev{});
+  kern<<<2 * pairs, Cfg<false, kWide>::kThreads, smem, stream>>>(ta, tb, tc, tc2, te, p, TpDev{});
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -87,7 +88,8 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   // can be described by a tensor map
   CUtensorMap tc = ta, tc2 = ta, te = ta;
   p.staged = 0;
-  if (!(a->flags & kGemmOutF32)) {
+  const int folds = ((a->flags & kGemmResidual) != 0) + ((a->flags & kGemmGeluDual) != 0) + ((a->flags & kGemmDGelu) != 0);
+  if (!(a->flags & kGemmOutF32) && folds <= 1) {      // combinations: direct stores
     auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld % 8 == 0; };
     bool ok = ok16(a->C, a->ldc);
     if (a->flags & kGemmGeluDual) ok = ok && ok16(a->C2, a->ldc);
@@ -102,11 +104,16 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
       p.staged = 1;
     }
   }
-  if ((a->flags & kGemmOutF32) && !(a->flags & (kGemmResidual | kGemmGeluDual | kGemmDGelu)) &&
-      (reinterpret_cast<uintptr_t>(a->C) & 15) == 0 && a->ldc % 4 == 0) {
-    rc = make_tmap_f32_2d(&tc, a->C, a->N, a->M, a->ldc, 32);
-    if (rc) return rc;
-    p.staged = 2;
+  // fp32 outputs the same way, a residual of fp32 among them (not under an accumulation, where each share would add it)
+  if ((a->flags & kGemmOutF32) && !(a->flags & (kGemmGeluDual | kGemmDGelu))) {
+    auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld % 4 == 0; };
+    const bool residual = a->flags & kGemmResidual;
+    if (ok16(a->C, a->ldc) && (!residual || (!(a->flags & (kGemmAtomic | kGemmAccum)) && ok16(a->residual, a->ldr)))) {
+      rc = make_tmap_f32_2d(&tc, a->C, a->N, a->M, a->ldc, 32);
+      if (!rc && residual) rc = make_tmap_f32_2d(&te, a->residual, a->N, a->M, a->ldr, 32);
+      if (rc) return rc;
+      p.staged = 2;
+    }
   }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -137,8 +144,13 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   const int total = p.tiles_m * p.tiles_n * split;
   const int pairs = total < max_pairs ? total : max_pairs;
   const bool amn = a->a_mn_major, bmn = a->b_mn_major;
-  if (!amn && !bmn) return launch<false, false>(ta, tb, tc, tc2, te, p, pairs, stream);
-  if (!amn && bmn) return launch<false, true>(ta, tb, tc, tc2, te, p, pairs, stream);
-  if (amn && bmn) return launch<true, true>(ta, tb, tc, tc2, te, p, pairs, stream);
-  return launch<true, false>(ta, tb, tc, tc2, te, p, pairs, stream);
+  auto go = [&](auto wide) {
+    constexpr bool kWide = decltype(wide)::value;
+    if (!amn && !bmn) return launch<false, false, kWide>(ta, tb, tc, tc2, te, p, pairs, stream);
+    if (!amn && bmn) return launch<false, true, kWide>(ta, tb, tc, tc2, te, p, pairs, stream);
+    if (amn && bmn) return launch<true, true, kWide>(ta, tb, tc, tc2, te, p, pairs, stream);
+    return launch<true, false, kWide>(ta, tb, tc, tc2, te, p, pairs, stream);
+  };
+  const bool wide = p.staged == 1 ? (a->flags & (kGemmGeluDual | kGemmDGelu)) : p.staged == 2 && (a->flags & kGemmResidual);
+  return wide ? go(std::true_type{}) : go(std::false_type{});
 }
