@@ -49,7 +49,7 @@ void kernel_status_reset() {
 
 // ------------------------------------------------------------------ GEMM
 // Kernel choice: 0 = one CTA per 128 x 256 tile, 1 = CTA pairs on 256 x 256 tiles.  An output whose 128 x 64 tiles
-// run all at once (itb_gemm_narrow) is computed by those in either mode.
+// run all at once (itb_gemm_is_small) is computed by those in either mode.
 int g_gemm_mode = 1;
 void set_gemm_mode(int64_t mode) { g_gemm_mode = static_cast<int>(mode); }
 int64_t get_gemm_mode() { return g_gemm_mode; }

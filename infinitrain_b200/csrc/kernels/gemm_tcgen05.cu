@@ -15,14 +15,13 @@
 //   wgrad     dW = dy^T x       A = dy [M,N] MN-major, B = x [M,K] MN-major (contraction M)
 //
 // Kernel shape: persistent, one CTA per SM, 192 threads = 1 TMA warp + 1 MMA warp + 4 epilogue
-// warps; tile 128 x BN x 64 with a ring of 4 stages in shared memory (BN 256) or 8 (BN 64) and two TMEM
-// accumulators so that the epilogue of tile i overlaps the main loop of tile i+1.
+// warps; tile 128 x 256 x 64 with a ring of 4 stages in shared memory and two TMEM accumulators so that the
+// epilogue of tile i overlaps the main loop of tile i+1.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <mutex>
-#include <type_traits>
 #include <unordered_map>
 
 #include "../common/ptx.cuh"
@@ -32,25 +31,25 @@
 namespace itb {
 
 constexpr int BM = 128;
+constexpr int BN = 256;
 constexpr int BK = 64;  // 64 bf16 = 128 bytes = one swizzle row
 constexpr int kGemmThreads = 192;
 
-template <int BN>
 struct SmemLayout {
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = BN * BK * 2;
-  static constexpr int kStages = BN == 64 ? 8 : 4;      // 192 KB either way
+  static constexpr int kStages = 4;                     // 192 KB
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kBarOffset = kStages * kStageBytes;
   // full[kStages], empty[kStages], tmem_full[2], tmem_empty[2], tmem holder, abort flag
   static constexpr int kTotal = kBarOffset + (2 * kStages + 4) * 8 + 16;
 };
 
-template <int BN, bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                          const __grid_constant__ CUtensorMap tma_b, const GemmDev p) {
-  using L = SmemLayout<BN>;
+  using L = SmemLayout;
   constexpr int kStages = L::kStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The dynamic shared window is only guaranteed 16-byte aligned: round up to 1024 (swizzle atom).
@@ -65,7 +64,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
 
   const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
-  constexpr uint32_t kTmemCols = 2 * BN;  // 128 or 512: a power of two >= 32
+  constexpr uint32_t kTmemCols = 2 * BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -367,11 +366,11 @@ static int num_sms() {
   return g_num_sms;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmDev& p, int grid,
                   cudaStream_t stream) {
-  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN>;
-  constexpr int smem = SmemLayout<BN>::kTotal + 1024;
+  auto kern = gemm_bf16_tcgen05_kernel<A_MN, B_MN>;
+  constexpr int smem = SmemLayout::kTotal + 1024;
   static PerDeviceOnce configured;
   if (configured.first()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -383,9 +382,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmDev& p
 
 }  // namespace itb
 
-extern "C" int itb_gemm_narrow(const ItbGemmArgs* a) {
+extern "C" int itb_gemm_is_small(const ItbGemmArgs* a) {
   const int other = kGemmAtomic | kGemmAccum | kGemmProbeNoLoad | kGemmProbeNoMma;
-  const long long tiles = static_cast<long long>((a->M + itb::BM - 1) / itb::BM) * ((a->N + 63) / 64);
+  const long long tiles = static_cast<long long>((a->M + 127) / 128) * ((a->N + 63) / 64);
   return !(a->flags & other) && tiles <= itb::num_sms();
 }
 
@@ -396,6 +395,7 @@ extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) ||
       (a->lda % 8) || (a->ldb % 8))
     return -2;
+  if (itb_gemm_is_small(a)) return itb_gemm_small(a, stream);
   CUtensorMap ta, tb;
   int rc;
   if (!a->a_mn_major)
@@ -403,16 +403,6 @@ extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
   else
     rc = make_tmap_bf16_2d(&ta, a->A, a->M, a->K, a->lda, 64, 64);
   if (rc) return rc;
-  // 128 x 64 tiles where they all run at once: a small output has too few 256-wide tiles to fill the machine (96 x 768
-  // has three), and each walks over the whole contraction by itself.
-  // 96 x 768 x 3072: 28.7 -> 19.5 us, 256 x 3072 x 768 (one CTA pair per 256 x 256 before): 16.4 -> 12.3 us, the
-  // forward and input-gradient GEMMs of GPT-2 124M on 4 x 64 tokens: 2.11 -> 1.38 ms.
-  // The line lies where these tiles need a second wave, which pairs need only from 75 tiles of 256 x 256 on.  Pairs
-  // against these tiles, us with the operands not in L2: 1152 x 1024 (144 tiles) at K 768 / 3072 / 8192 15.9 / 27.2 / 50.2
-  // against 12.3 / 20.5 / 39.0; 1153 x 1024 (160 tiles) 15.3 / 27.5 / 50.2 against 14.4 / 31.2 / 67.5; 2304 x 1024 (288)
-  // 16.5 / 28.7 / 54.1 against 15.2 / 32.7 / 69.6; 4096 x 1024 (512) 17.4 / 29.7 / 57.3 against 22.5 / 57.2 / 131.2.
-  const bool narrow = itb_gemm_narrow(a);
-  const int BN = narrow ? 64 : 256;
   if (!a->b_mn_major)
     rc = make_tmap_bf16_2d(&tb, a->B, a->K, a->N, a->ldb, 64, BN);
   else
@@ -455,12 +445,8 @@ extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
   const int total = p.tiles_m * p.tiles_n * split;
   const int grid = total < num_sms() ? total : num_sms();
   const bool amn = a->a_mn_major, bmn = a->b_mn_major;
-  auto go = [&](auto bn) {
-    constexpr int kBN = decltype(bn)::value;
-    if (!amn && !bmn) return launch<kBN, false, false>(ta, tb, p, grid, stream);
-    if (!amn && bmn) return launch<kBN, false, true>(ta, tb, p, grid, stream);
-    if (amn && bmn) return launch<kBN, true, true>(ta, tb, p, grid, stream);
-    return launch<kBN, true, false>(ta, tb, p, grid, stream);
-  };
-  return narrow ? go(std::integral_constant<int, 64>{}) : go(std::integral_constant<int, 256>{});
+  if (!amn && !bmn) return launch<false, false>(ta, tb, p, grid, stream);
+  if (!amn && bmn) return launch<false, true>(ta, tb, p, grid, stream);
+  if (amn && bmn) return launch<true, true>(ta, tb, p, grid, stream);
+  return launch<true, false>(ta, tb, p, grid, stream);
 }

@@ -54,7 +54,7 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) || (a->lda % 8) ||
       (a->ldb % 8))
     return -2;
-  if (itb_gemm_narrow(a)) return itb_gemm_bf16(a, stream);      // the same checks, the same flags
+  if (itb_gemm_is_small(a)) return itb_gemm_small(a, stream);
   CUtensorMap ta, tb;
   int rc;
   if (!a->a_mn_major)
