@@ -6,7 +6,10 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <array>
+#include <cmath>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "comm/comm.h"
@@ -124,19 +127,24 @@ void gemm(const at::Tensor& a, bool a_mn, const at::Tensor& b, bool b_mn, int64_
 }
 
 // ------------------------------------------------------------------ norms
+// `statistics`: what the backward pass needs; without it mean and rstd are undefined.
 std::vector<at::Tensor> layernorm_fwd(const at::Tensor& x, const at::Tensor& gamma,
                                       const c10::optional<at::Tensor>& beta, double eps,
-                                      at::ScalarType out_dtype) {
+                                      at::ScalarType out_dtype, bool statistics) {
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.is_contiguous(), "layernorm: contiguous input required");
   const int C = x.size(-1);
   const int rows = x.numel() / C;
   auto y = torch::empty_like(x, x.options().dtype(out_dtype));
-  auto mean = torch::empty({rows}, x.options().dtype(at::kFloat));
-  auto rstd = torch::empty({rows}, x.options().dtype(at::kFloat));
+  at::Tensor mean, rstd;
+  if (statistics) {
+    mean = torch::empty({rows}, x.options().dtype(at::kFloat));
+    rstd = torch::empty({rows}, x.options().dtype(at::kFloat));
+  }
   check_rc(itb_layernorm_fwd(x.data_ptr(), dt(x), gamma.data_ptr<float>(),
                              static_cast<const float*>(optr(beta)), y.data_ptr(), dt(y),
-                             mean.data_ptr<float>(), rstd.data_ptr<float>(), rows, C,
+                             statistics ? mean.data_ptr<float>() : nullptr,
+                             statistics ? rstd.data_ptr<float>() : nullptr, rows, C,
                              static_cast<float>(eps), cur_stream()),
            "layernorm_fwd");
   return {y, mean, rstd};
@@ -180,15 +188,16 @@ std::vector<at::Tensor> layernorm_bwd(const at::Tensor& dy, const at::Tensor& x,
   return {dx, dgamma, dbeta, dsum};
 }
 std::vector<at::Tensor> rmsnorm_fwd(const at::Tensor& x, const at::Tensor& gamma, double eps,
-                                    at::ScalarType out_dtype) {
+                                    at::ScalarType out_dtype, bool statistics) {
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.is_contiguous(), "rmsnorm: contiguous input required");
   const int C = x.size(-1);
   const int rows = x.numel() / C;
   auto y = torch::empty_like(x, x.options().dtype(out_dtype));
-  auto rstd = torch::empty({rows}, x.options().dtype(at::kFloat));
+  at::Tensor rstd;
+  if (statistics) rstd = torch::empty({rows}, x.options().dtype(at::kFloat));
   check_rc(itb_rmsnorm_fwd(x.data_ptr(), dt(x), gamma.data_ptr<float>(), y.data_ptr(), dt(y),
-                           rstd.data_ptr<float>(), rows, C, static_cast<float>(eps), cur_stream()),
+                           statistics ? rstd.data_ptr<float>() : nullptr, rows, C, static_cast<float>(eps), cur_stream()),
            "rmsnorm_fwd");
   return {y, rstd};
 }
@@ -477,6 +486,243 @@ void flash_attn_bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tenso
     check_rc(itb_flash_attn_bwd(&a, cur_stream()), "flash_attn_bwd");
 }
 
+// ------------------------------------------------------------------ whole passes of an op in one call
+// What an op's forward or backward does around its launches (shapes, strides, allocations) costs the host as much as the
+// launches themselves when each step is a call from Python: 87 ops on 1 x 96 tokens of GPT-2 124M took 2.3 ms of host time.
+using OptTensor = c10::optional<at::Tensor>;
+
+// `x` as a bf16 matrix whose rows TMA can read: unit column stride, rows and base on 16 bytes.
+at::Tensor bf16_rows(const at::Tensor& x) {
+  at::Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+  if (x2.scalar_type() != at::kBFloat16) x2 = x2.to(at::kBFloat16);
+  if (x2.stride(1) != 1 || (x2.stride(0) % 8) || (reinterpret_cast<uintptr_t>(x2.data_ptr()) % 16)) x2 = x2.contiguous();
+  if (x2.stride(0) % 8) {        // the gradient of a rank-4 product's rows are not a multiple of 16 bytes apart
+    const int64_t cols = x2.size(1);
+    at::Tensor padded = at::empty({x2.size(0), (cols + 7) / 8 * 8}, x2.options());
+    at::Tensor view = padded.narrow(1, 0, cols);
+    view.copy_(x2);
+    x2 = view;
+  }
+  return x2;
+}
+
+// The leading dimensions of `x` with `last` in the place of its last one.
+std::vector<int64_t> sizes_with_last(const at::Tensor& x, int64_t last) {
+  std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = last;
+  return sizes;
+}
+
+// A fresh output of `rows` x N, shaped like `x` but for its last dimension; its rows are `ld` elements apart.
+at::Tensor output_like(const at::Tensor& x, int64_t rows, int64_t N, int64_t ld, at::ScalarType dtype, void** data) {
+  if (ld == N) {
+    at::Tensor y = at::empty(sizes_with_last(x, N), x.options().dtype(dtype));
+    *data = y.data_ptr();
+    return y;
+  }
+  at::Tensor out = at::empty({rows, ld}, x.options().dtype(dtype));
+  *data = out.data_ptr();
+  return out.narrow(1, 0, N).view(sizes_with_last(x, N));
+}
+
+struct Gemm : ItbGemmArgs {
+  at::Tensor kept;        // a copy that the launch reads
+  Gemm(const at::Tensor& a, bool a_mn, const at::Tensor& b, bool b_mn, int64_t m, int64_t n, int64_t k) : ItbGemmArgs{} {
+    TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.device() == b.device(), "gemm: operands on one CUDA device required");
+    TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "gemm: bf16 operands required");
+    TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1,
+                "gemm: matrices with a contiguous innermost dimension required");
+    TORCH_CHECK(a_mn ? (a.size(0) == k && a.size(1) == m) : (a.size(0) == m && a.size(1) == k), "gemm: A shape mismatch");
+    TORCH_CHECK(b_mn ? (b.size(0) == k && b.size(1) == n) : (b.size(0) == n && b.size(1) == k), "gemm: B shape mismatch");
+    M = static_cast<int>(m), N = static_cast<int>(n), K = static_cast<int>(k);
+    A = a.data_ptr(), lda = a.stride(0), a_mn_major = a_mn;
+    B = b.data_ptr(), ldb = b.stride(0), b_mn_major = b_mn;
+    err = status_word(a.get_device()).data_ptr<int>();
+  }
+  Gemm& into(void* c, int64_t ld, int more_flags = 0) {
+    C = c, ldc = ld, flags |= more_flags;
+    return *this;
+  }
+  Gemm& add_bias(const OptTensor& b) {
+    if (b && b->defined()) {
+      TORCH_CHECK(b->is_cuda() && b->scalar_type() == at::kFloat && b->numel() >= N, "gemm: fp32 bias of length N required");
+      kept = b->contiguous();
+      bias = kept.data_ptr<float>();
+      flags |= kGemmBias;
+    }
+    return *this;
+  }
+  void run() {
+    if (g_gemm_mode == 1 && M > 128)
+      check_rc(itb_gemm_bf16_pair(this, cur_stream()), "gemm_bf16_tcgen05_pair");
+    else
+      check_rc(itb_gemm_bf16(this, cur_stream()), "gemm_bf16_tcgen05");
+  }
+};
+
+// Adds a residual to a GEMM's output (`keep` holds the matrix that the launch reads).
+void add_residual(Gemm& g, const OptTensor& residual, bool out_f32, at::Tensor* keep) {
+  if (!residual || !residual->defined()) return;
+  TORCH_CHECK(residual->scalar_type() == (out_f32 ? at::kFloat : at::kBFloat16), "gemm: residual must have C's dtype");
+  *keep = residual->reshape({g.M, g.N});
+  if (keep->stride(1) != 1) *keep = keep->contiguous();
+  g.residual = keep->data_ptr();
+  g.ldr = keep->stride(0);
+  g.flags |= kGemmResidual;
+}
+
+bool is_f32(const OptTensor& t) { return t && t->defined() && t->scalar_type() == at::kFloat; }
+
+// y = x w^T (+ bias) (+ residual) or gelu(x w^T + bias): {y, x as a matrix, pre-activation (rows padded to 64 elements)}
+std::tuple<at::Tensor, at::Tensor, OptTensor> linear_fwd(const at::Tensor& x, const at::Tensor& w, const OptTensor& bias,
+                                                         const OptTensor& residual, bool gelu) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t K = x.size(-1), N = w.size(0), ld = (N + 63) / 64 * 64;
+  at::Tensor x2 = bf16_rows(x), kept;
+  const int64_t M = x2.size(0);
+  const bool f32 = is_f32(residual);
+  Gemm g(x2, false, w, false, M, N, K);
+  void* data;
+  at::Tensor y = output_like(x, M, N, ld, f32 ? at::kFloat : at::kBFloat16, &data);
+  OptTensor pre;
+  g.add_bias(bias);
+  if (gelu) {
+    pre = at::empty({M, ld}, x2.options());
+    g.into(pre->data_ptr(), ld, kGemmGeluDual);
+    g.C2 = data;
+  } else {
+    g.into(data, ld, f32 ? kGemmOutF32 : 0);
+    add_residual(g, residual, f32, &kept);
+  }
+  g.run();
+  return {y, x2, pre};
+}
+
+// dW [N, K] = dy^T x in fp32, added to `main` (a slot of a flat gradient buffer) or as a fresh tensor.
+OptTensor weight_grad(const at::Tensor& dy2, const at::Tensor& x2, const OptTensor& main) {
+  const int64_t N = dy2.size(1), K = x2.size(1), M = x2.size(0);
+  OptTensor dw;
+  if (!main) dw = at::zeros({N, K}, dy2.options().dtype(at::kFloat));
+  const at::Tensor& out = main ? *main : *dw;
+  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kFloat && out.dim() == 2 && out.size(0) == N && out.size(1) >= K &&
+                  out.stride(1) == 1,
+              "linear: the weight's gradient slot must be an fp32 [N, K] matrix");
+  Gemm g(dy2, true, x2, true, N, K, M);
+  g.into(out.data_ptr(), out.stride(0), kGemmOutF32 | kGemmAtomic).run();
+  return dw;
+}
+
+// Column sums of dy, added to `main` or as a fresh tensor.  Matrices that the kernel cannot read are summed by torch, and
+// then not into `main`.
+OptTensor bias_grad(const at::Tensor& dy2, const OptTensor& main) {
+  if (dy2.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(dy2.data_ptr()) % 16 == 0) {
+    at::Tensor out = colsum(dy2, main);
+    return main ? OptTensor() : OptTensor(out);
+  }
+  return dy2.to(at::kFloat).sum(0);
+}
+
+// {dx, dw, db} of linear_fwd; what was added to a slot comes back as None.  `pre` (rows of any pitch) when the output went
+// through GELU, `w` when dx is wanted.
+std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const at::Tensor& dy, const at::Tensor& x2, const OptTensor& w,
+                                                       const OptTensor& pre, bool want_dw, const OptTensor& main_dw,
+                                                       bool want_db, const OptTensor& main_db) {
+  c10::cuda::CUDAGuard guard(dy.device());
+  at::Tensor dy2 = bf16_rows(dy);
+  const int64_t M = x2.size(0), N = dy2.size(1), K = x2.size(1);
+  if (pre) dy2 = bf16_rows(gelu_bwd(dy2.contiguous(), pre->narrow(1, 0, N).contiguous()));
+  OptTensor dx, dw, db;
+  if (w) {
+    dx = at::empty(sizes_with_last(dy, K), dy2.options());
+    Gemm(dy2, false, *w, true, M, K, N).into(dx->data_ptr(), K).run();
+  }
+  if (want_dw) dw = weight_grad(dy2, x2, main_dw);
+  if (want_db) db = bias_grad(dy2, main_db);
+  return {dx, dw, db};
+}
+
+// residual + gelu(x w_fc^T + b_fc) w_proj^T + b_proj: {y, x as a matrix, pre-activation, activation}
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> mlp_gelu_fwd(const at::Tensor& x, const at::Tensor& w_fc,
+                                                                        const OptTensor& b_fc, const at::Tensor& w_proj,
+                                                                        const OptTensor& b_proj, const OptTensor& residual) {
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor x2 = bf16_rows(x), kept;
+  const int64_t M = x2.size(0), C = x2.size(1), F = w_fc.size(0);
+  at::Tensor h = at::empty({M, F}, x2.options()), act = at::empty({M, F}, x2.options());
+  Gemm up(x2, false, w_fc, false, M, F, C);
+  up.add_bias(b_fc).into(h.data_ptr(), F, kGemmGeluDual);
+  up.C2 = act.data_ptr();
+  up.run();
+  const bool f32 = is_f32(residual);
+  at::Tensor y = at::empty(x.sizes(), x2.options().dtype(f32 ? at::kFloat : at::kBFloat16));
+  Gemm down(act, false, w_proj, false, M, C, F);
+  down.add_bias(b_proj).into(y.data_ptr(), C, f32 ? kGemmOutF32 : 0);
+  add_residual(down, residual, f32, &kept);
+  down.run();
+  return {y, x2, h, act};
+}
+
+// {dx, dw_fc, db_fc, dw_proj, db_proj}; see linear_bwd.
+std::tuple<OptTensor, OptTensor, OptTensor, OptTensor, OptTensor> mlp_gelu_bwd(
+    const at::Tensor& dy, const at::Tensor& x2, const at::Tensor& h, const at::Tensor& act, const at::Tensor& w_fc,
+    const at::Tensor& w_proj, bool want_dx, bool want_dw_fc, const OptTensor& main_fc, bool want_db_fc,
+    const OptTensor& main_b_fc, bool want_dw_proj, const OptTensor& main_proj, bool want_db_proj,
+    const OptTensor& main_b_proj) {
+  c10::cuda::CUDAGuard guard(dy.device());
+  at::Tensor dy2 = bf16_rows(dy);
+  const int64_t M = x2.size(0), C = x2.size(1), F = h.size(1);
+  at::Tensor dh = at::empty({M, F}, dy2.options());
+  Gemm g(dy2, false, w_proj, true, M, F, C);      // the derivative is applied in the epilogue
+  g.into(dh.data_ptr(), F, kGemmDGelu);
+  g.aux = h.data_ptr();
+  g.ld_aux = h.stride(0);
+  g.run();
+  OptTensor dx, dw_fc, db_fc, dw_proj, db_proj;
+  if (want_dw_proj) dw_proj = weight_grad(dy2, act, main_proj);
+  if (want_db_proj) db_proj = bias_grad(dy2, main_b_proj);
+  if (want_dx) {
+    dx = at::empty(sizes_with_last(dy, C), dy2.options());
+    Gemm(dh, false, w_fc, true, M, C, F).into(dx->data_ptr(), C).run();
+  }
+  if (want_dw_fc) dw_fc = weight_grad(dh, x2, main_fc);
+  if (want_db_fc) db_fc = bias_grad(dh, main_b_fc);
+  return {dx, dw_fc, db_fc, dw_proj, db_proj};
+}
+
+// Views of the query, key and value heads of a packed [B, T, (H + 2 KV) D] projection.
+std::array<at::Tensor, 3> packed_heads(const at::Tensor& qkv, int64_t H, int64_t KV, int64_t D) {
+  at::Tensor heads = qkv.view({qkv.size(0), qkv.size(1), H + 2 * KV, D});
+  return {heads.narrow(2, 0, H), heads.narrow(2, H, KV), heads.narrow(2, H + KV, KV)};
+}
+
+// Attention over a packed projection, with RoPE applied to it in place first: {o [B, T, H D], lse, the projection as
+// attention read it}
+std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_packed_fwd(const at::Tensor& packed, int64_t H, int64_t KV, int64_t D,
+                                                                    const OptTensor& freqs, int64_t pos0, bool causal) {
+  TORCH_CHECK(packed.dim() == 3, "attention: [B, T, (H + 2 KV) D] projection");
+  at::Tensor qkv = packed.scalar_type() == at::kBFloat16 ? packed : packed.to(at::kBFloat16);
+  if (freqs) {
+    if (!qkv.is_contiguous()) qkv = qkv.clone(at::MemoryFormat::Contiguous);      // (a transposed one keeps its order otherwise)
+    rope_inplace(qkv, *freqs, qkv.size(0), qkv.size(1), H + KV, D, qkv.stride(1), pos0, false);
+  }
+  auto [q, k, v] = packed_heads(qkv, H, KV, D);
+  std::vector<at::Tensor> out = flash_attn_fwd(q, k, v, 1.0 / std::sqrt(static_cast<double>(D)), causal);
+  return {out[0].view({qkv.size(0), qkv.size(1), H * D}), out[1], qkv};
+}
+
+at::Tensor attention_packed_bwd(const at::Tensor& dout, const at::Tensor& qkv, const at::Tensor& o, const at::Tensor& lse,
+                                int64_t H, int64_t KV, int64_t D, const OptTensor& freqs, int64_t pos0, bool causal) {
+  const int64_t B = qkv.size(0), T = qkv.size(1);
+  auto [q, k, v] = packed_heads(qkv, H, KV, D);
+  at::Tensor dqkv = at::empty_like(qkv);
+  auto [dq, dk, dv] = packed_heads(dqkv, H, KV, D);
+  at::Tensor d = dout.reshape({B, T, H, D});
+  if (d.scalar_type() != at::kBFloat16) d = d.to(at::kBFloat16);
+  flash_attn_bwd(d.contiguous(), q, k, v, o.view({B, T, H, D}), lse, dq, dk, dv, 1.0 / std::sqrt(static_cast<double>(D)), causal);
+  if (freqs) rope_inplace(dqkv, *freqs, B, T, H + KV, D, dqkv.stride(1), pos0, true);
+  return dqkv;
+}
+
 }  // namespace
 
 void bind_comm(pybind11::module_& m);
@@ -500,12 +746,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_attn_mode", &set_attn_mode);
   m.def("get_attn_mode", &get_attn_mode);
   m.def("get_gemm_mode", &get_gemm_mode);
-  m.def("layernorm_fwd", &layernorm_fwd);
+  m.def("layernorm_fwd", &layernorm_fwd, pybind11::arg("x"), pybind11::arg("gamma"), pybind11::arg("beta"),
+        pybind11::arg("eps"), pybind11::arg("out_dtype"), pybind11::arg("statistics") = true);
   m.def("layernorm_bwd", &layernorm_bwd, pybind11::arg("dy"), pybind11::arg("x"), pybind11::arg("gamma"),
         pybind11::arg("mean"), pybind11::arg("rstd"), pybind11::arg("has_beta"), pybind11::arg("dres") = pybind11::none(),
         pybind11::arg("dgamma_out") = pybind11::none(), pybind11::arg("dbeta_out") = pybind11::none(),
         pybind11::arg("dres_sum_out") = pybind11::none(), pybind11::arg("want_dres_sum") = false);
-  m.def("rmsnorm_fwd", &rmsnorm_fwd);
+  m.def("rmsnorm_fwd", &rmsnorm_fwd, pybind11::arg("x"), pybind11::arg("gamma"), pybind11::arg("eps"),
+        pybind11::arg("out_dtype"), pybind11::arg("statistics") = true);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, pybind11::arg("dy"), pybind11::arg("x"), pybind11::arg("gamma"), pybind11::arg("rstd"),
         pybind11::arg("dres") = pybind11::none(), pybind11::arg("dgamma_out") = pybind11::none(),
         pybind11::arg("dres_sum_out") = pybind11::none(), pybind11::arg("want_dres_sum") = false);
@@ -528,6 +776,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("colsum", &colsum, pybind11::arg("x"), pybind11::arg("into") = pybind11::none());
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd);
+  m.def("linear_fwd", &linear_fwd);
+  m.def("linear_bwd", &linear_bwd);
+  m.def("mlp_gelu_fwd", &mlp_gelu_fwd);
+  m.def("mlp_gelu_bwd", &mlp_gelu_bwd);
+  m.def("attention_packed_fwd", &attention_packed_fwd);
+  m.def("attention_packed_bwd", &attention_packed_bwd);
   bind_comm(m);
   bind_runtime(m);
 }

@@ -59,7 +59,7 @@ int itb_gemm_small(const ItbGemmArgs* args, cudaStream_t stream);
 int itb_gemm_bf16_pair(const ItbGemmArgs* args, cudaStream_t stream);
 
 // ------------------------------------------------------------------ normalisation
-// y = (x - mean) * rstd * gamma + beta over the last dimension C of [rows, C].
+// y = (x - mean) * rstd * gamma + beta over the last dimension C of [rows, C].  mean and rstd may be null: not stored.
 int itb_layernorm_fwd(const void* x, int x_dtype, const float* gamma, const float* beta, void* y,
                       int y_dtype, float* mean, float* rstd, int rows, int C, float eps,
                       cudaStream_t stream);

@@ -192,7 +192,7 @@ norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
     }
     if (lane == 0) {
       if (mean_out) mean_out[row] = mean;
-      rstd_out[row] = rstd;
+      if (rstd_out) rstd_out[row] = rstd;
     }
     auto emit = [&](int vi, float (&xv)[8]) {
       float g[8], o[8];

@@ -135,100 +135,70 @@ class _LinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, residual, gelu):
-        C = _C()
-        K = x.shape[-1]
-        N = weight.shape[0]
-        x2 = _as_bf16_2d(x)
-        M = x2.shape[0]
-        w = weight_lp(weight)
-        out_f32 = residual is not None and residual.dtype == torch.float32
-        ld = _pad_cols(N)
-        out = torch.empty((M, ld), device=x.device, dtype=torch.float32 if out_f32 else torch.bfloat16)
-        flags = 0
-        if out_f32:
-            flags |= C.GEMM_OUT_F32
-        if bias is not None:
-            flags |= C.GEMM_BIAS
-        res2 = None
-        if residual is not None:
-            res2 = residual.reshape(M, N)
-            if res2.stride(-1) != 1:
-                res2 = res2.contiguous()
-            flags |= C.GEMM_RESIDUAL
-        pre = None
-        if gelu:
-            assert residual is None, "gelu and residual epilogues are not combined"
-            pre = torch.empty((M, ld), device=x.device, dtype=torch.bfloat16)
-            flags |= C.GEMM_GELU_DUAL
-            C.gemm(x2, False, w, False, M, N, K, pre, out, bias, None, None, flags, 0)
-        else:
-            C.gemm(x2, False, w, False, M, N, K, out, None, bias, res2, None, flags, 0)
+        assert not gelu or residual is None, "gelu and residual epilogues are not combined"
+        y, x2, pre = _C().linear_fwd(x, weight_lp(weight), bias, residual, gelu)
         _counters["launches"] += 1
-        ctx.save_for_backward(x2, weight, pre if gelu else None)
-        ctx.bias_param = bias            # the Parameter itself: its gradient may go straight to a flat buffer
-        ctx.bias_elsewhere = claim_bias_grad(residual, bias)
-        ctx.has_bias = bias is not None
-        ctx.has_res = residual is not None
-        ctx.gelu = gelu
-        ctx.x_shape = x.shape
-        ctx.x_dtype = x.dtype
-        ctx.res_dtype = residual.dtype if residual is not None else None
-        ctx.N, ctx.K, ctx.M, ctx.ld = N, K, M, ld
-        y = out[:, :N] if ld != N else out
-        return y.view(*x.shape[:-1], N)
+        ctx.save_for_backward(x2, weight, pre)
+        # the Parameter itself: its gradient may go straight to a flat buffer
+        ctx.meta = (bias, claim_bias_grad(residual, bias), x.dtype, residual.dtype if residual is not None else None)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        C = _C()
         x2, weight, pre = ctx.saved_tensors
-        M, N, K = ctx.M, ctx.N, ctx.K
-        d_res = dy if ctx.has_res else None
-        if d_res is not None and d_res.dtype != ctx.res_dtype:
-            d_res = d_res.to(ctx.res_dtype)
-        dy2 = _as_bf16_2d(dy)
-        if ctx.gelu:
-            # dy is the gradient of the activation output: fold gelu'(h) in with one pointwise pass.
-            dyc = dy2 if dy2.is_contiguous() else dy2.contiguous()
-            prec = pre[:, :N] if ctx.ld != N else pre
-            prec = prec if prec.is_contiguous() else prec.contiguous()
-            dy2 = _as_bf16_2d(C.gelu_bwd(dyc, prec))
-            _counters["launches"] += 1
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            w = weight_lp(weight)
-            dx2 = torch.empty((M, K), device=dy.device, dtype=torch.bfloat16)
-            C.gemm(dy2, False, w, True, M, K, N, dx2, None, None, None, None, 0, 0)
-            _counters["launches"] += 1
-            dx = dx2.view(ctx.x_shape)
-            if ctx.x_dtype != torch.bfloat16:
-                dx = dx.to(ctx.x_dtype)
-        if ctx.needs_input_grad[1]:
-            dw = _wgrad(C, dy2, x2, weight, N, K, M)
-        if ctx.has_bias and ctx.needs_input_grad[2] and not ctx.bias_elsewhere:
-            db = _bias_grad(C, dy2, N, ctx.bias_param)
-        return dx, dw, db, d_res, None
+        bias, bias_elsewhere, x_dtype, res_dtype = ctx.meta
+        need_x, need_w, need_b = ctx.needs_input_grad[:3]
+        d_res = None
+        if res_dtype is not None:
+            d_res = dy if dy.dtype == res_dtype else dy.to(res_dtype)
+        need_b = need_b and bias is not None and not bias_elsewhere
+        main_w = _weight_slot(weight) if need_w else None
+        main_b = _main_grad_of(bias) if need_b else None
+        # with GELU dy is the gradient of the activation: gelu'(h) is folded in with one pointwise pass
+        dx, dw, db = _C().linear_bwd(dy, x2, weight_lp(weight) if need_x else None, pre, need_w, main_w, need_b, main_b)
+        _counters["launches"] += (pre is not None) + need_x + need_w + (need_w and main_w is None) + 2 * need_b
+        if dx is not None and x_dtype != torch.bfloat16:
+            dx = dx.to(x_dtype)
+        return dx, _weight_done(weight, need_w, dw), _bias_done(bias, need_b, db), d_res, None
+
+
+def _weight_slot(weight):
+    """The fp32 tensor that ``weight``'s gradient is added to by the kernel (flat DDP / ZeRO gradient buffers), or None."""
+    if getattr(weight, "_itb_shared", False):
+        # A parameter used by several ops (tied embedding / head) receives the rest of its gradient
+        # through autograd; its ready hook must fire once, after the last contribution.
+        return None
+    main = getattr(weight, "main_grad", None)
+    if main is None and getattr(weight, "_itb_main_grad_fn", None) is not None:
+        main = weight._itb_main_grad_fn()
+    return main
+
+
+def _weight_done(weight, wanted, dw):
+    """What autograd gets for ``weight``: ``dw``, or None after its grad-ready hooks when the kernel has added it."""
+    if not wanted:
+        return None
+    if dw is None:
+        for hook in getattr(weight, "_itb_grad_ready_hooks", ()):
+            hook(weight)
+        return None
+    return dw if weight.dtype == torch.float32 else dw.to(weight.dtype)
+
+
+def _bias_done(bias, wanted, db):
+    if wanted and db is None:
+        _grad_written(bias)
+    return db
 
 
 def _wgrad(C, dy2, x2, weight, N, K, M):
     """dW[N,K] = dy^T x in fp32.  Accumulates straight into ``weight.main_grad`` when the parameter
     has one (flat DDP / ZeRO gradient buffers) and then fires its grad-ready hooks."""
-    main = getattr(weight, "main_grad", None)
-    if main is None and getattr(weight, "_itb_main_grad_fn", None) is not None:
-        main = weight._itb_main_grad_fn()
-    if getattr(weight, "_itb_shared", False):
-        # A parameter used by several ops (tied embedding / head) receives the rest of its gradient
-        # through autograd; its ready hook must fire once, after the last contribution.
-        main = None
-    if main is not None:
-        C.gemm(dy2, True, x2, True, N, K, M, main, None, None, None, None, C.GEMM_OUT_F32 | C.GEMM_ATOMIC, 0)
-        _counters["launches"] += 1
-        for hook in getattr(weight, "_itb_grad_ready_hooks", ()):
-            hook(weight)
-        return None
-    dw = torch.zeros((N, K), device=dy2.device, dtype=torch.float32)
+    main = _weight_slot(weight)
+    dw = main if main is not None else torch.zeros((N, K), device=dy2.device, dtype=torch.float32)
     C.gemm(dy2, True, x2, True, N, K, M, dw, None, None, None, None, C.GEMM_OUT_F32 | C.GEMM_ATOMIC, 0)
-    _counters["launches"] += 2
-    return dw if weight.dtype == torch.float32 else dw.to(weight.dtype)
+    _counters["launches"] += 1 + (main is None)
+    return _weight_done(weight, True, None if main is not None else dw)
 
 
 def _main_grad_of(p: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -300,62 +270,35 @@ class _MlpGeluFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w_fc, b_fc, w_proj, b_proj, residual):
-        C = _C()
-        Cd = x.shape[-1]
-        F = w_fc.shape[0]
-        x2 = _as_bf16_2d(x)
-        M = x2.shape[0]
-        wfc, wpr = weight_lp(w_fc), weight_lp(w_proj)
-        h = torch.empty((M, F), device=x.device, dtype=torch.bfloat16)
-        g = torch.empty((M, F), device=x.device, dtype=torch.bfloat16)
-        flags = C.GEMM_GELU_DUAL | (C.GEMM_BIAS if b_fc is not None else 0)
-        C.gemm(x2, False, wfc, False, M, F, Cd, h, g, b_fc, None, None, flags, 0)
-        out_f32 = residual is not None and residual.dtype == torch.float32
-        out = torch.empty((M, Cd), device=x.device, dtype=torch.float32 if out_f32 else torch.bfloat16)
-        flags = (C.GEMM_OUT_F32 if out_f32 else 0) | (C.GEMM_BIAS if b_proj is not None else 0)
-        res2 = None
-        if residual is not None:
-            res2 = residual.reshape(M, Cd)
-            res2 = res2 if res2.stride(-1) == 1 else res2.contiguous()
-            flags |= C.GEMM_RESIDUAL
-        C.gemm(g, False, wpr, False, M, Cd, F, out, None, b_proj, res2, None, flags, 0)
+        y, x2, h, g = _C().mlp_gelu_fwd(x, weight_lp(w_fc), b_fc, weight_lp(w_proj), b_proj, residual)
         _counters["launches"] += 2
         ctx.save_for_backward(x2, h, g, w_fc, w_proj)
-        ctx.bias_params = (b_fc, b_proj)
-        ctx.bias_elsewhere = claim_bias_grad(residual, b_proj)
-        ctx.meta = (M, Cd, F, x.shape, x.dtype, b_fc is not None, b_proj is not None,
-                    residual.dtype if residual is not None else None)
-        return out.view(x.shape)
+        ctx.meta = (b_fc, b_proj, claim_bias_grad(residual, b_proj), x.dtype, residual.dtype if residual is not None else None)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        C = _C()
         x2, h, g, w_fc, w_proj = ctx.saved_tensors
-        M, Cd, F, x_shape, x_dtype, has_bfc, has_bpr, res_dtype = ctx.meta
+        b_fc, b_proj, bias_elsewhere, x_dtype, res_dtype = ctx.meta
+        need_x, need_fc, need_bfc, need_proj, need_bproj = ctx.needs_input_grad[:5]
         d_res = None
         if res_dtype is not None:
             d_res = dy if dy.dtype == res_dtype else dy.to(res_dtype)
-        dy2 = _as_bf16_2d(dy)
-        # dh = (dy Wproj) * gelu'(h): derivative applied in the GEMM epilogue.
-        dh = torch.empty((M, F), device=dy.device, dtype=torch.bfloat16)
-        C.gemm(dy2, False, weight_lp(w_proj), True, M, F, Cd, dh, None, None, None, h, C.GEMM_DGELU, 0)
-        _counters["launches"] += 1
-        dw_proj = _wgrad(C, dy2, g, w_proj, Cd, F, M) if ctx.needs_input_grad[3] else None
-        b_fc, b_proj = ctx.bias_params
-        db_proj = None
-        if has_bpr and ctx.needs_input_grad[4] and not ctx.bias_elsewhere:
-            db_proj = _bias_grad(C, dy2, Cd, b_proj)
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx2 = torch.empty((M, Cd), device=dy.device, dtype=torch.bfloat16)
-            C.gemm(dh, False, weight_lp(w_fc), True, M, Cd, F, dx2, None, None, None, None, 0, 0)
-            _counters["launches"] += 1
-            dx = dx2.view(x_shape)
-            if x_dtype != torch.bfloat16:
-                dx = dx.to(x_dtype)
-        dw_fc = _wgrad(C, dh, x2, w_fc, F, Cd, M) if ctx.needs_input_grad[1] else None
-        db_fc = _bias_grad(C, dh, F, b_fc) if has_bfc and ctx.needs_input_grad[2] else None
-        return dx, dw_fc, db_fc, dw_proj, db_proj, d_res
+        need_bfc = need_bfc and b_fc is not None
+        need_bproj = need_bproj and b_proj is not None and not bias_elsewhere
+        main_fc = _weight_slot(w_fc) if need_fc else None
+        main_proj = _weight_slot(w_proj) if need_proj else None
+        dx, dw_fc, db_fc, dw_proj, db_proj = _C().mlp_gelu_bwd(
+            dy, x2, h, g, weight_lp(w_fc), weight_lp(w_proj), need_x, need_fc, main_fc, need_bfc,
+            _main_grad_of(b_fc) if need_bfc else None, need_proj, main_proj, need_bproj,
+            _main_grad_of(b_proj) if need_bproj else None)
+        _counters["launches"] += (1 + need_x + need_fc + (need_fc and main_fc is None) + need_proj
+                                  + (need_proj and main_proj is None) + 2 * need_bfc + 2 * need_bproj)
+        if dx is not None and x_dtype != torch.bfloat16:
+            dx = dx.to(x_dtype)
+        dw_proj = _weight_done(w_proj, need_proj, dw_proj)
+        db_proj = _bias_done(b_proj, need_bproj, db_proj)
+        return dx, _weight_done(w_fc, need_fc, dw_fc), _bias_done(b_fc, need_bfc, db_fc), dw_proj, db_proj, d_res
 
 
 def mlp_gelu(x, w_fc, b_fc, w_proj, b_proj, residual=None):
@@ -417,7 +360,7 @@ class _LayerNormFn(torch.autograd.Function):
     def forward(ctx, x, gamma, beta, eps, out_dtype, holder=None):
         C = _C()
         xc = x if x.is_contiguous() else x.contiguous()
-        y, mean, rstd = C.layernorm_fwd(xc, gamma, beta, eps, out_dtype)
+        y, mean, rstd = C.layernorm_fwd(xc, gamma, beta, eps, out_dtype, type(ctx) is not _NoContext)
         _counters["launches"] += 1
         ctx.save_for_backward(xc, mean, rstd)
         ctx.params = (gamma, beta)
@@ -453,7 +396,7 @@ class _RMSNormFn(torch.autograd.Function):
     def forward(ctx, x, gamma, eps, out_dtype, holder=None):
         C = _C()
         xc = x if x.is_contiguous() else x.contiguous()
-        y, rstd = C.rmsnorm_fwd(xc, gamma, eps, out_dtype)
+        y, rstd = C.rmsnorm_fwd(xc, gamma, eps, out_dtype, type(ctx) is not _NoContext)
         _counters["launches"] += 1
         ctx.save_for_backward(xc, rstd)
         ctx.params = (gamma,)
@@ -645,40 +588,18 @@ class _AttentionFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, H, KV, D, freqs, pos0, causal):
-        C = _C()
-        B, T, _ = qkv.shape
-        if qkv.dtype != torch.bfloat16:
-            qkv = qkv.to(torch.bfloat16)
-        if freqs is not None:
-            qkv = qkv.clone() if not qkv.is_contiguous() else qkv
-            C.rope_inplace(qkv, freqs, B, T, H + KV, D, qkv.stride(1), pos0, False)
-            _counters["launches"] += 1
-        q, k, v = _heads(qkv, H, KV, D)
-        scale = 1.0 / math.sqrt(D)
-        o, lse = C.flash_attn_fwd(q, k, v, scale, causal)
-        _counters["launches"] += 1
+        o, lse, qkv = _C().attention_packed_fwd(qkv, H, KV, D, freqs, pos0, causal)
+        _counters["launches"] += 1 + (freqs is not None)
         ctx.save_for_backward(qkv, o, lse, freqs)
-        ctx.meta = (H, KV, D, pos0, causal, scale)
-        return o.view(B, T, H * D)
+        ctx.meta = (H, KV, D, pos0, causal)
+        return o
 
     @staticmethod
     def backward(ctx, dout):
-        C = _C()
         qkv, o, lse, freqs = ctx.saved_tensors
-        H, KV, D, pos0, causal, scale = ctx.meta
-        B, T, _ = qkv.shape
-        q, k, v = _heads(qkv, H, KV, D)
-        dqkv = torch.empty_like(qkv)
-        dq, dk, dv = _heads(dqkv, H, KV, D)
-        do = dout.reshape(B, T, H, D)
-        if do.dtype != torch.bfloat16:
-            do = do.to(torch.bfloat16)
-        do = do if do.is_contiguous() else do.contiguous()
-        C.flash_attn_bwd(do, q, k, v, o, lse, dq, dk, dv, scale, causal)
-        _counters["launches"] += 4
-        if freqs is not None:
-            C.rope_inplace(dqkv, freqs, B, T, H + KV, D, dqkv.stride(1), pos0, True)
-            _counters["launches"] += 1
+        H, KV, D, pos0, causal = ctx.meta
+        dqkv = _C().attention_packed_bwd(dout, qkv, o, lse, H, KV, D, freqs, pos0, causal)
+        _counters["launches"] += 4 + (freqs is not None)
         return dqkv, None, None, None, None, None, None
 
 

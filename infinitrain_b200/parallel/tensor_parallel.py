@@ -30,6 +30,8 @@ def _seq_dim(x: torch.Tensor) -> int:
 
 
 def _tp() -> Optional[ProcessGroup]:
+    if genv.GlobalEnv.Instance().tensor_parallel_size == 1:
+        return None         # asked several times an op: not by way of the group's name
     g = tp_group()
     return g if (g is not None and g.world_size > 1) else None
 
@@ -209,17 +211,19 @@ class ColumnParallelLinear(Module):
         from . import symm
 
         add_bias = self.bias if (self.has_bias and not self.skip_bias_add) else None
+        if _tp() is None:       # the region functions would be identities
+            y = ops.linear(x, self.weight, add_bias, gelu=gelu)
+            return (y, self.bias) if self.skip_bias_add else y
         if self.sequence_parallel and symm.fused_tp_enabled(x):
             symm.note_tp_path(self, x, True)
             y = symm.allgather_linear(x, self.weight, add_bias, gelu=gelu)
-        elif (not self.sequence_parallel and not self.input_is_parallel and _tp() is not None
+        elif (not self.sequence_parallel and not self.input_is_parallel
               and symm.fused_tp_enabled(x, seq_sharded=False)):
             # replicated input: no communication forward, the gradient all-reduce is fused into dgrad
             symm.note_tp_path(self, x, True)
             y = symm.copy_linear(x, self.weight, add_bias, gelu=gelu)
         else:
-            if _tp() is not None:
-                symm.note_tp_path(self, x, False)
+            symm.note_tp_path(self, x, False)
             if self.sequence_parallel:
                 x = GatherFromSPRegionFunc(x)
             elif not self.input_is_parallel:
@@ -262,10 +266,10 @@ class RowParallelLinear(Module):
         one tensor-parallel rank it is fused into the GEMM epilogue."""
         from . import symm
 
-        if not self.input_is_parallel:
+        grp = _tp()
+        if grp is not None and not self.input_is_parallel:
             x = ScatterToTPRegionFunc(x)
         add_bias = self.bias if (self.has_bias and not self.skip_bias_add) else None
-        grp = _tp()
         if grp is None or not self.reduce_output:
             y = ops.linear(x, self.weight, add_bias, residual=residual)
         elif self.sequence_parallel and symm.fused_tp_enabled(x, seq_sharded=False):
