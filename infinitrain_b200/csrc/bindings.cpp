@@ -602,13 +602,13 @@ std::tuple<at::Tensor, at::Tensor, OptTensor> linear_fwd(const at::Tensor& x, co
 OptTensor weight_grad(const at::Tensor& dy2, const at::Tensor& x2, const OptTensor& main) {
   const int64_t N = dy2.size(1), K = x2.size(1), M = x2.size(0);
   OptTensor dw;
-  if (!main) dw = at::zeros({N, K}, dy2.options().dtype(at::kFloat));
+  if (!main) dw = at::empty({N, K}, dy2.options().dtype(at::kFloat));
   const at::Tensor& out = main ? *main : *dw;
   TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kFloat && out.dim() == 2 && out.size(0) == N && out.size(1) >= K &&
                   out.stride(1) == 1,
               "linear: the weight's gradient slot must be an fp32 [N, K] matrix");
   Gemm g(dy2, true, x2, true, N, K, M);
-  g.into(out.data_ptr(), out.stride(0), kGemmOutF32 | kGemmAtomic).run();
+  g.into(out.data_ptr(), out.stride(0), kGemmOutF32 | kGemmAtomic | (main ? 0 : kGemmFresh)).run();
   return dw;
 }
 
@@ -732,6 +732,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "infinitrain_b200 native layer (sm_100a kernels, NVLink kernels, host runtime)";
   m.attr("GEMM_OUT_F32") = static_cast<int>(kGemmOutF32);
   m.attr("GEMM_ATOMIC") = static_cast<int>(kGemmAtomic);
+  m.attr("GEMM_FRESH") = static_cast<int>(kGemmFresh);
   m.attr("GEMM_ACCUM") = static_cast<int>(kGemmAccum);
   m.attr("GEMM_BIAS") = static_cast<int>(kGemmBias);
   m.attr("GEMM_RESIDUAL") = static_cast<int>(kGemmResidual);

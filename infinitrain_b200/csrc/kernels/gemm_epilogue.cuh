@@ -30,6 +30,19 @@ struct GemmDev {
                        // 16-byte aligned bases and row pitches); 0: direct stores from registers
 };
 
+// The output of a GEMM that sums into something new (kGemmFresh): cleared if several shares of the contraction are added to
+// it, or there is nothing to contract; otherwise the flags lose the addition and the one share is stored.
+// (A fresh 128256 x 2048 weight gradient was cleared, read and written: 1.05 GB each way three times instead of once.)
+static inline cudaError_t prepare_fresh_output(const ItbGemmArgs* a, int split, int* flags, cudaStream_t stream) {
+  if ((a->flags & (kGemmFresh | kGemmAtomic)) != (kGemmFresh | kGemmAtomic)) return cudaSuccess;
+  if (split == 1 && a->K > 0) {
+    *flags &= ~kGemmAtomic;
+    return cudaSuccess;
+  }
+  if (a->M <= 0 || a->N <= 0) return cudaSuccess;
+  return cudaMemset2DAsync(a->C, static_cast<size_t>(a->ldc) * 4, 0, static_cast<size_t>(a->N) * 4, a->M, stream);
+}
+
 // One MUFU instruction; relative error about 2^-11, below bf16 resolution.
 __device__ __forceinline__ float tanh_fast(float x) {
   float y;

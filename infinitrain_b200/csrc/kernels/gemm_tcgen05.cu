@@ -390,7 +390,10 @@ extern "C" int itb_gemm_is_small(const ItbGemmArgs* a) {
 
 extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
   using namespace itb;
-  if (a->M <= 0 || a->N <= 0 || a->K <= 0) return 0;
+  if (a->M <= 0 || a->N <= 0 || a->K <= 0) {
+    int flags = a->flags;
+    return static_cast<int>(prepare_fresh_output(a, 1, &flags, stream));
+  }
   // TMA needs 16-byte aligned bases and row strides.
   if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) ||
       (a->lda % 8) || (a->ldb % 8))
@@ -442,6 +445,8 @@ extern "C" int itb_gemm_bf16(const ItbGemmArgs* a, cudaStream_t stream) {
     split = (p.k_blocks + per - 1) / per;
   }
   p.split_k = split;
+  const cudaError_t fresh = prepare_fresh_output(a, split, &p.flags, stream);
+  if (fresh != cudaSuccess) return static_cast<int>(fresh);
   const int total = p.tiles_m * p.tiles_n * split;
   const int grid = total < num_sms() ? total : num_sms();
   const bool amn = a->a_mn_major, bmn = a->b_mn_major;

@@ -50,7 +50,10 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
 extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   using namespace itb;
   using namespace itb::pair;
-  if (a->M <= 0 || a->N <= 0 || a->K <= 0) return 0;
+  if (a->M <= 0 || a->N <= 0 || a->K <= 0) {
+    int flags = a->flags;
+    return static_cast<int>(prepare_fresh_output(a, 1, &flags, stream));
+  }
   if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) || (a->lda % 8) ||
       (a->ldb % 8))
     return -2;
@@ -141,6 +144,8 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
     split = (p.k_blocks + per - 1) / per;
   }
   p.split_k = split;
+  const cudaError_t fresh = prepare_fresh_output(a, split, &p.flags, stream);
+  if (fresh != cudaSuccess) return static_cast<int>(fresh);
   const int total = p.tiles_m * p.tiles_n * split;
   const int pairs = total < max_pairs ? total : max_pairs;
   const bool amn = a->a_mn_major, bmn = a->b_mn_major;
