@@ -22,12 +22,19 @@ constexpr int kMaxPartialRows = 592;    // 4 blocks per SM on 148 SMs
 #define ITB_NORM_FWD_BLOCKS_PER_SM 8
 #endif
 constexpr int kNormFwdBlocksPerSm = ITB_NORM_FWD_BLOCKS_PER_SM;
-// warp-per-row backward: two sets of packed row chunks (current and prefetched) beside the per-lane
-// parameter-gradient accumulators need more than 168 registers
-#ifndef ITB_NORM_BWD_BLOCKS_PER_SM
-#define ITB_NORM_BWD_BLOCKS_PER_SM 2
-#endif
-constexpr int kNormBwdBlocksPerSm = ITB_NORM_BWD_BLOCKS_PER_SM;
+// Backward: what a thread holds of a row in registers (two sets, current and prefetched, where that leaves room), and how
+// many blocks an SM then takes.  A row's way through a block is a chain (loads, two sums across the lanes, stores), so the
+// loads of the next row run under it; without that rows of 2048 and more waited for memory every time (2048 x 2048 bf16:
+// 38.0 -> 27.7 us with the reduction of the parameter gradients, 4096 x 4096: 81.0 -> 56.4), although four blocks shared an SM.
+template <typename TDY, typename TX, typename TDX, bool kRms, int kChunks, bool kRes, bool kWide>
+struct BwdShape {
+  static constexpr int kRaw = kChunks * 2 * static_cast<int>(sizeof(TDY) + sizeof(TX) + (kRes ? sizeof(TDX) : 0));
+  static constexpr int kHeld = kChunks * 8 * (2 + !kRms + kRes);       // gamma and the parameter gradients
+  static constexpr bool kPrefetch = !kWide || 2 * kRaw + kHeld <= 192;
+  // four blocks of 128 threads have 128 registers a thread, three 168: with fewer than they need the rows spill
+  static constexpr int kRegisters = kRaw * (kPrefetch ? 2 : 1) + kHeld + 40;
+  static constexpr int kBlocksPerSm = !kWide ? 2 : kChunks == 1 ? 4 : kPrefetch ? 2 : kRegisters <= 128 ? 4 : kRegisters <= 168 ? 3 : 2;
+};
 
 template <typename T>
 __device__ __forceinline__ float to_f(T v);
@@ -235,7 +242,7 @@ norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
 // the stream past the norm (the skip connection); its column sums come out as a third partial row
 // (they are the bias gradient of the projection that wrote into the stream).
 //
-// kWide = false: one warp per row (rows up to 1024 wide), kChunks chunks of 8 per lane.
+// kWide = false: one warp per row (rows up to 768 wide, many of them), kChunks chunks of 8 per lane.
 // kWide = true:  the whole block works on one row at a time (rows up to kChunks * 1024 wide); the two
 //                row statistics cross the warps through a double-buffered shared-memory slot, one
 //                __syncthreads per row.
@@ -244,7 +251,8 @@ norm_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ gamma,
 // the warps add their registers to a shared-memory row in turns; in the wide layout every thread owns
 // its columns.
 template <typename TDY, typename TX, typename TDX, bool kRms, int kChunks, bool kRes, bool kWide>
-__global__ void __launch_bounds__(kNormThreads, kWide ? 4 : kNormBwdBlocksPerSm)
+__global__ void
+__launch_bounds__(kNormThreads, (BwdShape<TDY, TX, TDX, kRms, kChunks, kRes, kWide>::kBlocksPerSm))
 norm_bwd_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x,
                 const float* __restrict__ gamma, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const TDX* __restrict__ dres,
@@ -269,9 +277,8 @@ norm_bwd_kernel(const TDY* __restrict__ dy, const TX* __restrict__ x,
   }
   const int row_step = kWide ? static_cast<int>(gridDim.x) : static_cast<int>(gridDim.x) * kNormWarps;
   int parity = 0;
-  // The loads of the NEXT row are issued before the current row's arithmetic (kPrefetch: the
-  // warp-per-row layout, where the register budget allows a second set of packed chunks).
-  constexpr bool kPrefetch = !kWide;
+  // kPrefetch: the loads of the NEXT row are issued before the current row's arithmetic.
+  constexpr bool kPrefetch = BwdShape<TDY, TX, TDX, kRms, kChunks, kRes, kWide>::kPrefetch;
   Raw8<TDY> rd[kChunks], nd[kPrefetch ? kChunks : 1];
   Raw8<TX> rx[kChunks], nx[kPrefetch ? kChunks : 1];
   Raw8<TDX> rres[kRes ? kChunks : 1], nres[(kRes && kPrefetch) ? kChunks : 1];
@@ -457,6 +464,8 @@ partial_reduce_kernel(const float* __restrict__ partial, int prow_stride, int nr
   out[oc] = ((accumulate >> which) & 1) ? out[oc] + t : t;
 }
 
+constexpr int kWarpRowsFrom = 4096;      // rows up to 768 wide: more than this many go one to a warp
+
 // Upper bound of the backward grid for `rows` rows in either layout: what callers size `partial` with.
 static int norm_grid(int rows) { return rows < kMaxPartialRows ? (rows < 1 ? 1 : rows) : kMaxPartialRows; }
 static int norm_bwd_grid(int rows, bool wide, int blocks_per_sm) {
@@ -514,17 +523,25 @@ static int norm_bwd_dispatch(const void* dy, int dyd, const void* x, int xd, con
                              int accumulate, cudaStream_t s) {
   if (C % 8 || C > 6144) return -3;
   if (rows < 1) return 0;
-  const bool wide = C > 1024;
-  const int grid = norm_bwd_grid(rows, wide, wide ? 4 : kNormBwdBlocksPerSm);
-  const int smem = wide ? 2 * kNormWarps * 2 * static_cast<int>(sizeof(float)) : 3 * C * static_cast<int>(sizeof(float));
+  // One warp per row keeps a row's sums inside the warp, but pays at the end for warps that add their parameter gradients up
+  // in turns, and 128 columns a warp past 768 take a fourth chunk and its registers.  us with a warp / a block per row,
+  // bf16 with a residual's gradient: 96 x 768 21.4 / 13.0, 2331 x 768 23.6 / 21.6, 4096 x 768 25.6 / 25.5, 8192 x 768 31.7 / 31.7,
+  // 16384 x 768 42.1 / 46.0, 8192 x 1024 58.3 / 35.8.
+  const bool wide = C > 768 || rows <= kWarpRowsFrom;
+  int grid = 0;
 #define LAUNCH_K(TDY, TX, TDX, CH, RES, WIDE)                                                     \
-  norm_bwd_kernel<TDY, TX, TDX, kRms, CH, RES, WIDE><<<grid, kNormThreads, smem, s>>>(            \
-      static_cast<const TDY*>(dy), static_cast<const TX*>(x), gamma, mean, rstd,                  \
-      static_cast<const TDX*>(dres), static_cast<TDX*>(dx), partial, rows, C)
+  do {                                                                                            \
+    constexpr int smem_wide = 2 * kNormWarps * 2 * static_cast<int>(sizeof(float));               \
+    grid = norm_bwd_grid(rows, WIDE, BwdShape<TDY, TX, TDX, kRms, CH, RES, WIDE>::kBlocksPerSm);  \
+    norm_bwd_kernel<TDY, TX, TDX, kRms, CH, RES, WIDE>                                            \
+        <<<grid, kNormThreads, WIDE ? smem_wide : 3 * C * static_cast<int>(sizeof(float)), s>>>(  \
+            static_cast<const TDY*>(dy), static_cast<const TX*>(x), gamma, mean, rstd,            \
+            static_cast<const TDX*>(dres), static_cast<TDX*>(dx), partial, rows, C);              \
+  } while (0)
 #define LAUNCH_R(TDY, TX, TDX, RES)                                  \
   do {                                                               \
-    if (C <= 768) LAUNCH_K(TDY, TX, TDX, 3, RES, false);             \
-    else if (C <= 1024) LAUNCH_K(TDY, TX, TDX, 4, RES, false);       \
+    if (!wide) LAUNCH_K(TDY, TX, TDX, 3, RES, false);                \
+    else if (C <= 1024) LAUNCH_K(TDY, TX, TDX, 1, RES, true);        \
     else if (C <= 2048) LAUNCH_K(TDY, TX, TDX, 2, RES, true);        \
     else if (C <= 4096) LAUNCH_K(TDY, TX, TDX, 4, RES, true);        \
     else LAUNCH_K(TDY, TX, TDX, 6, RES, true);                       \
