@@ -53,8 +53,7 @@ typedef struct {
 int itb_gemm_bf16(const ItbGemmArgs* args, cudaStream_t stream);
 // Whether the output is small enough for 128 x 64 tiles to run all at once (and nothing is accumulated) ...
 int itb_gemm_is_small(const ItbGemmArgs* args);
-// ... and the kernel for it (gemm_small.cu), to which the other two entries hand such outputs.  split_k: into how many
-// shares (1, 2, 4, 8) the contraction is dealt out, 0 = choose.
+// ... and the kernel for it (gemm_small.cu), to which the other two entries hand such outputs.  split_k is not looked at.
 int itb_gemm_small(const ItbGemmArgs* args, cudaStream_t stream);
 // Same contract, computed by CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair) unless the output is that small.
 int itb_gemm_bf16_pair(const ItbGemmArgs* args, cudaStream_t stream);
