@@ -62,8 +62,8 @@ __device__ __forceinline__ float dgelu_tanh(float x) {
   constexpr float k0 = 0.7978845608028654f, k1 = 0.044715f;
   const float x2 = x * x;
   const float t = tanh_fast(x * fmaf(x2, k0 * k1, k0));
-  const float du = x * fmaf(x2, 1.5f * k0 * k1, 0.5f * k0);      // 0.5 x u'
-  return fmaf(fmaf(-t, t, 1.f), du, fmaf(0.5f, t, 0.5f));
+  // 0.5 x u' meets 1 - t^2 one factor at a time: whole it is infinite from 2e13 on, where 1 - t^2 is zero
+  return fmaf(fmaf(-t, t, 1.f) * x, fmaf(x2, 1.5f * k0 * k1, 0.5f * k0), fmaf(0.5f, t, 0.5f));
 }
 
 // v: 32 consecutive accumulator columns [col0, col0 + 32) of output row `row`.

@@ -66,3 +66,19 @@ def test_epilogue_over_several_tiles(M, N, K, kind):
         assert ((out2[:, :N].double() - act).abs() <= unit * act.abs() + 1e-6 * K + 2.0 ** -11 * got.abs()).all()
     if not f32:         # bulk stores end on 16 bytes; nothing is written beyond
         assert torch.isnan(out[:, (N + 7) // 8 * 8:].float()).all()
+
+
+@pytest.mark.parametrize("M", [64, 40960])        # 128 x 64 tiles, CTA pairs
+def test_gelu_derivative_far_from_zero(M):
+    """1 and 0 as far as the square of the input is finite: the cube is not from 7e12 on."""
+    from infinitrain_b200 import _ext
+
+    C = _ext.load(required=True)
+    one = torch.zeros(M, 64, device="cuda", dtype=torch.bfloat16)
+    one[:, 0] = 1
+    far = torch.logspace(1, 19, 32, device="cuda")
+    h = torch.cat((far, -far)).bfloat16().expand(M, 64).contiguous()
+    out = torch.full((M, 64), float("nan"), device="cuda", dtype=torch.bfloat16)
+    C.gemm(one, False, one[:64], False, M, 64, 64, out, None, None, None, h, C.GEMM_DGELU, 0)      # the product is 1
+    assert torch.equal(out, (h > 0).bfloat16())
+    assert C.kernel_status() == 0
