@@ -598,8 +598,15 @@ std::tuple<at::Tensor, at::Tensor, OptTensor> linear_fwd(const at::Tensor& x, co
   return {y, x2, pre};
 }
 
+// Called as soon as the kernel that adds a gradient to its slot has been launched, ahead of the pass's other launches, so
+// that a reduction of the bucket the gradient completes starts under them; nothing when it is None.
+using Ready = pybind11::object;
+void call(const Ready& ready) {
+  if (!ready.is_none()) ready();
+}
+
 // dW [N, K] = dy^T x in fp32, added to `main` (a slot of a flat gradient buffer) or as a fresh tensor.
-OptTensor weight_grad(const at::Tensor& dy2, const at::Tensor& x2, const OptTensor& main) {
+OptTensor weight_grad(const at::Tensor& dy2, const at::Tensor& x2, const OptTensor& main, const Ready& ready) {
   const int64_t N = dy2.size(1), K = x2.size(1), M = x2.size(0);
   OptTensor dw;
   if (!main) dw = at::empty({N, K}, dy2.options().dtype(at::kFloat));
@@ -609,15 +616,18 @@ OptTensor weight_grad(const at::Tensor& dy2, const at::Tensor& x2, const OptTens
               "linear: the weight's gradient slot must be an fp32 [N, K] matrix");
   Gemm g(dy2, true, x2, true, N, K, M);
   g.into(out.data_ptr(), out.stride(0), kGemmOutF32 | kGemmAtomic | (main ? 0 : kGemmFresh)).run();
+  if (main) call(ready);
   return dw;
 }
 
 // Column sums of dy, added to `main` or as a fresh tensor.  Matrices that the kernel cannot read are summed by torch, and
 // then not into `main`.
-OptTensor bias_grad(const at::Tensor& dy2, const OptTensor& main) {
+OptTensor bias_grad(const at::Tensor& dy2, const OptTensor& main, const Ready& ready) {
   if (dy2.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(dy2.data_ptr()) % 16 == 0) {
     at::Tensor out = colsum(dy2, main);
-    return main ? OptTensor() : OptTensor(out);
+    if (!main) return out;
+    call(ready);
+    return {};
   }
   return dy2.to(at::kFloat).sum(0);
 }
@@ -626,7 +636,8 @@ OptTensor bias_grad(const at::Tensor& dy2, const OptTensor& main) {
 // through GELU, `w` when dx is wanted.
 std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const at::Tensor& dy, const at::Tensor& x2, const OptTensor& w,
                                                        const OptTensor& pre, bool want_dw, const OptTensor& main_dw,
-                                                       bool want_db, const OptTensor& main_db) {
+                                                       const Ready& dw_ready, bool want_db, const OptTensor& main_db,
+                                                       const Ready& db_ready) {
   c10::cuda::CUDAGuard guard(dy.device());
   at::Tensor dy2 = bf16_rows(dy);
   const int64_t M = x2.size(0), N = dy2.size(1), K = x2.size(1);
@@ -636,8 +647,8 @@ std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const at::Tensor& dy, con
     dx = at::empty(sizes_with_last(dy, K), dy2.options());
     Gemm(dy2, false, *w, true, M, K, N).into(dx->data_ptr(), K).run();
   }
-  if (want_dw) dw = weight_grad(dy2, x2, main_dw);
-  if (want_db) db = bias_grad(dy2, main_db);
+  if (want_dw) dw = weight_grad(dy2, x2, main_dw, dw_ready);
+  if (want_db) db = bias_grad(dy2, main_db, db_ready);
   return {dx, dw, db};
 }
 
@@ -665,9 +676,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> mlp_gelu_fwd(const at
 // {dx, dw_fc, db_fc, dw_proj, db_proj}; see linear_bwd.
 std::tuple<OptTensor, OptTensor, OptTensor, OptTensor, OptTensor> mlp_gelu_bwd(
     const at::Tensor& dy, const at::Tensor& x2, const at::Tensor& h, const at::Tensor& act, const at::Tensor& w_fc,
-    const at::Tensor& w_proj, bool want_dx, bool want_dw_fc, const OptTensor& main_fc, bool want_db_fc,
-    const OptTensor& main_b_fc, bool want_dw_proj, const OptTensor& main_proj, bool want_db_proj,
-    const OptTensor& main_b_proj) {
+    const at::Tensor& w_proj, bool want_dx, bool want_dw_fc, const OptTensor& main_fc, const Ready& fc_ready,
+    bool want_db_fc, const OptTensor& main_b_fc, const Ready& b_fc_ready, bool want_dw_proj, const OptTensor& main_proj,
+    const Ready& proj_ready, bool want_db_proj, const OptTensor& main_b_proj, const Ready& b_proj_ready) {
   c10::cuda::CUDAGuard guard(dy.device());
   at::Tensor dy2 = bf16_rows(dy);
   const int64_t M = x2.size(0), C = x2.size(1), F = h.size(1);
@@ -678,14 +689,14 @@ std::tuple<OptTensor, OptTensor, OptTensor, OptTensor, OptTensor> mlp_gelu_bwd(
   g.ld_aux = h.stride(0);
   g.run();
   OptTensor dx, dw_fc, db_fc, dw_proj, db_proj;
-  if (want_dw_proj) dw_proj = weight_grad(dy2, act, main_proj);
-  if (want_db_proj) db_proj = bias_grad(dy2, main_b_proj);
+  if (want_dw_proj) dw_proj = weight_grad(dy2, act, main_proj, proj_ready);
+  if (want_db_proj) db_proj = bias_grad(dy2, main_b_proj, b_proj_ready);
   if (want_dx) {
     dx = at::empty(sizes_with_last(dy, C), dy2.options());
     Gemm(dh, false, w_fc, true, M, C, F).into(dx->data_ptr(), C).run();
   }
-  if (want_dw_fc) dw_fc = weight_grad(dh, x2, main_fc);
-  if (want_db_fc) db_fc = bias_grad(dh, main_b_fc);
+  if (want_dw_fc) dw_fc = weight_grad(dh, x2, main_fc, fc_ready);
+  if (want_db_fc) db_fc = bias_grad(dh, main_b_fc, b_fc_ready);
   return {dx, dw_fc, db_fc, dw_proj, db_proj};
 }
 

@@ -10,6 +10,7 @@ bf16 between the fused kernels.
 """
 from __future__ import annotations
 
+import functools
 import math
 from typing import Optional
 
@@ -155,11 +156,12 @@ class _LinearFn(torch.autograd.Function):
         main_w = _weight_slot(weight, ctx, 1) if need_w else None
         main_b = _main_grad_of(bias) if need_b else None
         # with GELU dy is the gradient of the activation: gelu'(h) is folded in with one pointwise pass
-        dx, dw, db = _C().linear_bwd(dy, x2, weight_lp(weight) if need_x else None, pre, need_w, main_w, need_b, main_b)
+        dx, dw, db = _C().linear_bwd(dy, x2, weight_lp(weight) if need_x else None, pre, need_w, main_w, _ready(weight, main_w),
+                                     need_b, main_b, _ready(bias, main_b))
         _counters["launches"] += (pre is not None) + need_x + need_w + 2 * need_b
         if dx is not None and x_dtype != torch.bfloat16:
             dx = dx.to(x_dtype)
-        return dx, _weight_done(weight, need_w, dw), _bias_done(bias, need_b, db), d_res, None
+        return dx, _for_autograd(weight, dw), db, d_res, None
 
 
 def _weight_slot(weight, ctx=None, index=0):
@@ -193,21 +195,16 @@ def _accumulated_slot(ctx, index, p):
         return None
 
 
-def _weight_done(weight, wanted, dw):
-    """What autograd gets for ``weight``: ``dw``, or None after its grad-ready hooks when the kernel has added it."""
-    if not wanted:
+def _ready(p, slot):
+    """What a native pass calls once it has launched the kernel that adds ``p``'s gradient to ``slot``, or None."""
+    if slot is None or not (getattr(p, "_itb_grad_ready_hooks", None) or getattr(p, "_itb_grad_elsewhere", False)):
         return None
-    if dw is None:
-        for hook in getattr(weight, "_itb_grad_ready_hooks", ()):
-            hook(weight)
-        return None
-    return dw if weight.dtype == torch.float32 else dw.to(weight.dtype)
+    return functools.partial(_grad_written, p)
 
 
-def _bias_done(bias, wanted, db):
-    if wanted and db is None:
-        _grad_written(bias)
-    return db
+def _for_autograd(weight, dw):
+    """``dw`` (None when the kernel has added it) in the type of ``weight``."""
+    return dw if dw is None or weight.dtype == torch.float32 else dw.to(weight.dtype)
 
 
 def _wgrad(C, dy2, x2, weight, N, K, M):
@@ -218,7 +215,10 @@ def _wgrad(C, dy2, x2, weight, N, K, M):
     flags = C.GEMM_OUT_F32 | C.GEMM_ATOMIC | (C.GEMM_FRESH if main is None else 0)
     C.gemm(dy2, True, x2, True, N, K, M, dw, None, None, None, None, flags, 0)
     _counters["launches"] += 1
-    return _weight_done(weight, True, None if main is not None else dw)
+    if main is None:
+        return _for_autograd(weight, dw)
+    _grad_written(weight)
+    return None
 
 
 def _main_grad_of(p: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -308,16 +308,16 @@ class _MlpGeluFn(torch.autograd.Function):
         need_bproj = need_bproj and b_proj is not None and not bias_elsewhere
         main_fc = _weight_slot(w_fc) if need_fc else None
         main_proj = _weight_slot(w_proj) if need_proj else None
+        main_bfc = _main_grad_of(b_fc) if need_bfc else None
+        main_bproj = _main_grad_of(b_proj) if need_bproj else None
         dx, dw_fc, db_fc, dw_proj, db_proj = _C().mlp_gelu_bwd(
-            dy, x2, h, g, weight_lp(w_fc), weight_lp(w_proj), need_x, need_fc, main_fc, need_bfc,
-            _main_grad_of(b_fc) if need_bfc else None, need_proj, main_proj, need_bproj,
-            _main_grad_of(b_proj) if need_bproj else None)
+            dy, x2, h, g, weight_lp(w_fc), weight_lp(w_proj), need_x, need_fc, main_fc, _ready(w_fc, main_fc),
+            need_bfc, main_bfc, _ready(b_fc, main_bfc), need_proj, main_proj, _ready(w_proj, main_proj),
+            need_bproj, main_bproj, _ready(b_proj, main_bproj))
         _counters["launches"] += 1 + need_x + need_fc + need_proj + 2 * need_bfc + 2 * need_bproj
         if dx is not None and x_dtype != torch.bfloat16:
             dx = dx.to(x_dtype)
-        dw_proj = _weight_done(w_proj, need_proj, dw_proj)
-        db_proj = _bias_done(b_proj, need_bproj, db_proj)
-        return dx, _weight_done(w_fc, need_fc, dw_fc), _bias_done(b_fc, need_bfc, db_fc), dw_proj, db_proj, d_res
+        return dx, _for_autograd(w_fc, dw_fc), db_fc, _for_autograd(w_proj, dw_proj), db_proj, d_res
 
 
 def mlp_gelu(x, w_fc, b_fc, w_proj, b_proj, residual=None):

@@ -80,3 +80,50 @@ def test_fresh_weight_gradient(rows, N, K, mode):
     finally:
         C.set_gemm_mode(old)
     assert C.kernel_status() == 0
+
+
+def _slot_with_hook(shape, name, log, later):
+    """A parameter whose ready hook notes which of the slots in ``later`` still hold nothing at its place in the stream."""
+    p = torch.nn.Parameter(torch.randn(shape, device="cuda") * 0.1)
+    p.main_grad = torch.zeros_like(p.detach())
+    later.append(p.main_grad)
+    p._itb_grad_ready_hooks = [lambda q: log.append((name, p.main_grad.clone(), [s.clone() for s in later]))]
+    return p
+
+
+@pytest.mark.parametrize("op", ["linear", "linear_gelu", "mlp"])
+def test_ready_hooks_run_between_the_launches(op):
+    """A hook runs as soon as its own gradient has been launched, ahead of the kernels of the gradients that follow."""
+    log, slots = [], []
+    x = torch.randn(2, 40, 64, device="cuda").bfloat16().requires_grad_()
+    make = lambda shape, name: _slot_with_hook(shape, name, log, slots)
+    if op == "mlp":
+        w_fc, b_fc, w_proj, b_proj = make((128, 64), "w_fc"), make((128,), "b_fc"), make((64, 128), "w_proj"), make((64,), "b_proj")
+        order, places = ["w_proj", "b_proj", "w_fc", "b_fc"], [2, 3, 0, 1]
+        run = lambda: F.mlp_gelu(x, w_fc, b_fc, w_proj, b_proj)
+    else:
+        w, b = make((72, 64), "w"), make((72,), "b")
+        order, places = ["w", "b"], [0, 1]
+        run = lambda: F.linear(x, w, b, gelu=op == "linear_gelu")
+    with AutocastGuard(DeviceType.kCUDA, DataType.kBFLOAT16):
+        y = run()
+    y.backward(torch.randn_like(y))
+    assert [name for name, _, _ in log] == order
+    for k, (name, own, seen) in enumerate(log):
+        assert torch.equal(own, slots[places[k]]) and own.any(), name          # written whole when the hook runs
+        for later in places[k + 1:]:
+            assert not seen[later].any(), (name, "ran after", order[places.index(later)])
+
+
+def test_error_in_a_ready_hook_is_the_callers():
+    w = torch.nn.Parameter(torch.randn(72, 64, device="cuda"))
+    w.main_grad = torch.zeros_like(w.detach())
+
+    def fail(p):
+        raise KeyError("bucket")
+
+    w._itb_grad_ready_hooks = [fail]
+    x = torch.randn(40, 64, device="cuda").bfloat16()
+    y = F.linear(x, w)
+    with pytest.raises(KeyError, match="bucket"):
+        y.backward(torch.randn_like(y))
