@@ -303,6 +303,12 @@ void embedding_bwd(const at::Tensor& idx, const at::Tensor& dout,
                    int64_t pos0, int64_t vocab_start) {
   c10::cuda::CUDAGuard guard(dout.device());
   TORCH_CHECK(dout.is_contiguous() && dout.dim() == 3, "embedding_bwd: contiguous [B,T,C]");
+  auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  TORCH_CHECK(aligned(dout), "embedding_bwd: a gradient on a 16-byte boundary");
+  for (const auto* table : {&dwte, &dwpe})
+    TORCH_CHECK(!table->has_value() || ((*table)->is_cuda() && (*table)->scalar_type() == at::kFloat && (*table)->dim() >= 2 &&
+                                        (*table)->size(-1) == dout.size(2) && (*table)->is_contiguous() && aligned(**table)),
+                "embedding_bwd: contiguous fp32 tables as wide as the gradient, on a 16-byte boundary");
   const int B = dout.size(0), T = dout.size(1), C = dout.size(2);
   int64_t vend = vocab_start + (dwte.has_value() ? dwte->size(0) : 0);
   check_rc(itb_embedding_bwd(reinterpret_cast<const long long*>(idx.data_ptr<int64_t>()),
@@ -571,6 +577,19 @@ void add_residual(Gemm& g, const OptTensor& residual, bool out_f32, at::Tensor* 
   g.flags |= kGemmResidual;
 }
 
+// Whether a kernel may add the gradient of the leaf `p` to `slot` in autograd's place: `slot` is its whole .grad, in fp32 and
+// on the boundary that the kernels' vector accesses need, and no hook of the leaf or of its accumulator waits for the sum.
+bool adds_in_place(const at::Tensor& p, const at::Tensor& slot) {
+  const at::Tensor& grad = p.grad();
+  if (!grad.defined() || grad.data_ptr() != slot.data_ptr() || slot.scalar_type() != at::kFloat ||
+      grad.scalar_type() != at::kFloat || slot.sizes() != p.sizes() || grad.sizes() != p.sizes() || !slot.is_contiguous() ||
+      !grad.is_contiguous() || reinterpret_cast<uintptr_t>(slot.data_ptr()) % 16)
+    return false;
+  const auto node = torch::autograd::impl::try_get_grad_accumulator(p);
+  return !node || (node->tensor_pre_hooks().empty() && node->pre_hooks().empty() && node->post_hooks().empty() &&
+                   !node->tensor_post_acc_grad_hooks());
+}
+
 bool is_f32(const OptTensor& t) { return t && t->defined() && t->scalar_type() == at::kFloat; }
 
 // y = x w^T (+ bias) (+ residual) or gelu(x w^T + bias): {y, x as a matrix, pre-activation (rows padded to 64 elements)}
@@ -788,6 +807,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("colsum", &colsum, pybind11::arg("x"), pybind11::arg("into") = pybind11::none());
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd);
+  m.def("adds_in_place", &adds_in_place);
   m.def("linear_fwd", &linear_fwd);
   m.def("linear_bwd", &linear_bwd);
   m.def("mlp_gelu_fwd", &mlp_gelu_fwd);

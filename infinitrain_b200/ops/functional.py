@@ -179,14 +179,12 @@ def _weight_slot(weight, ctx=None, index=0):
 def _accumulated_slot(ctx, index, p):
     """The fp32 tensor that autograd would add the gradient of ``p`` to, the input of ``ctx``'s node whose edge is
     ``index``, when nobody looks at that gradient on its way there: a kernel may add to the tensor itself and hand nothing on.
-    (The tied 50257 x 768 table of GPT-2: two gradients cleared, two additions, 0.26 ms a step.)  None with hooks, with
-    another ``.grad`` than the slot, in a pass that asks for the gradient itself (``torch.autograd.grad``) or leaves
+    (The tied 50257 x 768 table of GPT-2: two gradients cleared, two additions, 0.26 ms a step.)  None with hooks (of the
+    tensor or of its accumulator node), with another ``.grad`` than the slot or one off the 16-byte grid, in a pass that asks for the gradient itself (``torch.autograd.grad``) or leaves
     ``p`` out, and while the pass is recorded."""
     main = getattr(p, "main_grad", None)
-    if (main is None or main.dtype != torch.float32 or not main.is_contiguous() or torch.is_grad_enabled()
-            or p.grad is None or p.grad.data_ptr() != main.data_ptr() or getattr(p, "_itb_grad_ready_hooks", None)
-            or getattr(p, "_itb_sp_hooked", False) or getattr(p, "_backward_hooks", None)
-            or getattr(p, "_post_accumulate_grad_hooks", None)):
+    if (main is None or torch.is_grad_enabled() or getattr(p, "_itb_grad_ready_hooks", None)
+            or getattr(p, "_itb_sp_hooked", False) or not _C().adds_in_place(p, main)):
         return None
     node = ctx.next_functions[index][0]
     try:
@@ -659,6 +657,8 @@ class _EmbeddingFn(torch.autograd.Function):
         idx, wte, wpe = ctx.saved_tensors
         pos0, vocab_start = ctx.meta
         dout = dout if dout.is_contiguous() else dout.contiguous()
+        if dout.data_ptr() % 16:
+            dout = dout.clone()
         # the kernel adds: to the tables' own gradients where it may, else to cleared ones that autograd adds on
         slots = [None, None]
         grads = [None, None]
@@ -666,7 +666,7 @@ class _EmbeddingFn(torch.autograd.Function):
             if table is not None and ctx.needs_input_grad[1 + i]:
                 slots[i] = _accumulated_slot(ctx, 1 + i, table)
                 if slots[i] is None:
-                    slots[i] = grads[i] = torch.zeros_like(table, dtype=torch.float32)
+                    slots[i] = grads[i] = torch.zeros_like(table, dtype=torch.float32, memory_format=torch.contiguous_format)
         C.embedding_bwd(idx, dout, *slots, pos0, vocab_start)
         _counters["launches"] += sum(s is not None for s in slots) + sum(g is not None for g in grads)
         return None, *grads, None, None, None

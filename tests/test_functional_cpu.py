@@ -239,3 +239,37 @@ def test_print_options_apply_to_print():
         assert "..." in buf.getvalue()
     finally:
         T.SetPrintOptions(profile="default", sci_mode=None)
+
+
+@pytest.mark.parametrize("how", ["plain", "offset", "other_grad", "no_grad", "half", "transposed", "hook", "post_hook", "node_prehook",
+                                 "node_hook"])
+def test_slot_that_a_kernel_may_add_to(how):
+    """Only the leaf's whole fp32 gradient on the 16-byte grid that the kernels' vector accesses need, with nobody waiting
+    for the sum; decided on the host, nothing is launched."""
+    from infinitrain_b200 import _ext
+
+    C = _ext.load(required=False)
+    if C is None:
+        pytest.skip("native extension not built")
+    p = torch.nn.Parameter(torch.randn(6, 8))
+    slot = torch.zeros(49)[1:].view(6, 8) if how == "offset" else torch.zeros(6, 8)
+    assert slot.data_ptr() % 16 == (4 if how == "offset" else 0)
+    accumulator = p.expand_as(p).grad_fn.next_functions[0][0]
+    if how != "no_grad":
+        p.grad = torch.zeros(6, 8) if how == "other_grad" else slot
+    if how == "half":
+        p.grad = None
+        p.data = p.data.bfloat16()
+        p.grad = slot.view(torch.bfloat16)[:, :8]      # the same address
+        assert p.grad.data_ptr() == slot.data_ptr()
+    elif how == "transposed":
+        p.grad = slot.view(8, 6).t()
+    elif how == "hook":
+        p.register_hook(lambda g: g)
+    elif how == "post_hook":
+        p.register_post_accumulate_grad_hook(lambda q: None)
+    elif how == "node_prehook":
+        accumulator.register_prehook(lambda g: None)
+    elif how == "node_hook":
+        accumulator.register_hook(lambda gi, go: None)
+    assert C.adds_in_place(p, slot) == (how == "plain")

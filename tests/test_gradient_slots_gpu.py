@@ -127,3 +127,24 @@ def test_error_in_a_ready_hook_is_the_callers():
     y = F.linear(x, w)
     with pytest.raises(KeyError, match="bucket"):
         y.backward(torch.randn_like(y))
+
+
+def test_hook_of_the_accumulator_sees_the_gradient():
+    """Hooks of the node that adds a table's gradient up (what a wrapper for data parallelism registers) get it whole."""
+    table = _leaf((100, 64), True)
+    node = table.expand_as(table).grad_fn.next_functions[0][0]
+    seen = []
+    node.register_prehook(lambda grads: seen.append(grads[0]))
+    F.embedding(torch.randint(0, 100, (2, 16), device="cuda"), table).sum().backward()
+    assert len(seen) == 1 and seen[0] is not None and torch.equal(seen[0], table.grad) and table.grad.any()
+
+
+def test_embedding_gradient_off_the_16_byte_grid():
+    """A gradient whose rows start anywhere is copied before the kernel reads it."""
+    table = _leaf((100, 64), False)
+    idx = torch.randint(0, 100, (2, 16), device="cuda")
+    dout = torch.randn(2 * 16 * 64 + 1, device="cuda")[1:].view(2, 16, 64)
+    assert dout.is_contiguous() and dout.data_ptr() % 16
+    (got,) = torch.autograd.grad(F.embedding(idx, table), table, dout)
+    want = torch.zeros(100, 64, device="cuda").index_add_(0, idx.flatten(), dout.view(-1, 64))
+    assert (got - want).norm() <= 1e-6 * want.norm()
