@@ -56,6 +56,9 @@ int itb_gemm_is_small(const ItbGemmArgs* args);
 // ... and the kernel for it (gemm_small.cu), to which the other two entries hand such outputs.  split_k is not looked at.
 int itb_gemm_small(const ItbGemmArgs* args, cudaStream_t stream);
 // Same contract, computed by CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair) unless the output is that small.
+// Where C (and C2) are on 16 bytes with rows a multiple of 16 bytes apart, a row's last bulk store writes its 16 bytes whole:
+// zeros in the columns from N to the next multiple of 8 (bf16) or 4 (fp32), which have to belong to the buffer.  Not so with
+// an fp32 residual or an accumulation, which leave what is there.
 int itb_gemm_bf16_pair(const ItbGemmArgs* args, cudaStream_t stream);
 
 // ------------------------------------------------------------------ normalisation

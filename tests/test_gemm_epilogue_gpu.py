@@ -64,8 +64,10 @@ def test_epilogue_over_several_tiles(M, N, K, kind):
     if kind.startswith("gelu"):
         act = torch.nn.functional.gelu(got, approximate="tanh")
         assert ((out2[:, :N].double() - act).abs() <= unit * act.abs() + 1e-6 * K + 2.0 ** -11 * got.abs()).all()
-    if not f32:         # bulk stores end on 16 bytes; nothing is written beyond
-        assert torch.isnan(out[:, (N + 7) // 8 * 8:].float()).all()
+    # bulk stores of bf16 end on 16 bytes; nothing is written beyond, and beyond N by fp32 with a residual or a sum
+    end = N if f32 else (N + 7) // 8 * 8
+    for o in (out, out2) if kind.startswith("gelu") else (out,):
+        assert (o[:, end:] == 2.0).all() if kind == "add" else torch.isnan(o[:, end:].float()).all()
 
 
 @pytest.mark.parametrize("M", [64, 40960])        # 128 x 64 tiles, CTA pairs
