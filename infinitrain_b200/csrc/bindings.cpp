@@ -497,11 +497,15 @@ void flash_attn_bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tenso
 // launches themselves when each step is a call from Python: 87 ops on 1 x 96 tokens of GPT-2 124M took 2.3 ms of host time.
 using OptTensor = c10::optional<at::Tensor>;
 
+// Whether the rows of a matrix are one row expanded (the gradient of a sum over rows): a tensor map needs a pitch.
+bool one_row(const at::Tensor& x) { return x.size(0) > 1 && x.stride(0) == 0; }
+
 // `x` as a bf16 matrix whose rows TMA can read: unit column stride, rows and base on 16 bytes.
 at::Tensor bf16_rows(const at::Tensor& x) {
   at::Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
   if (x2.scalar_type() != at::kBFloat16) x2 = x2.to(at::kBFloat16);
-  if (x2.stride(1) != 1 || (x2.stride(0) % 8) || (reinterpret_cast<uintptr_t>(x2.data_ptr()) % 16)) x2 = x2.contiguous();
+  if (x2.stride(1) != 1 || one_row(x2) || (x2.stride(0) % 8) || (reinterpret_cast<uintptr_t>(x2.data_ptr()) % 16))
+    x2 = x2.contiguous();
   if (x2.stride(0) % 8) {        // the gradient of a rank-4 product's rows are not a multiple of 16 bytes apart
     const int64_t cols = x2.size(1);
     at::Tensor padded = at::empty({x2.size(0), (cols + 7) / 8 * 8}, x2.options());
@@ -571,7 +575,7 @@ void add_residual(Gemm& g, const OptTensor& residual, bool out_f32, at::Tensor* 
   if (!residual || !residual->defined()) return;
   TORCH_CHECK(residual->scalar_type() == (out_f32 ? at::kFloat : at::kBFloat16), "gemm: residual must have C's dtype");
   *keep = residual->reshape({g.M, g.N});
-  if (keep->stride(1) != 1) *keep = keep->contiguous();
+  if (keep->stride(1) != 1 || one_row(*keep)) *keep = keep->contiguous();
   g.residual = keep->data_ptr();
   g.ldr = keep->stride(0);
   g.flags |= kGemmResidual;
@@ -807,6 +811,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("colsum", &colsum, pybind11::arg("x"), pybind11::arg("into") = pybind11::none());
   m.def("flash_attn_fwd", &flash_attn_fwd);
   m.def("flash_attn_bwd", &flash_attn_bwd);
+  m.def("bf16_rows", &bf16_rows);
   m.def("adds_in_place", &adds_in_place);
   m.def("linear_fwd", &linear_fwd);
   m.def("linear_bwd", &linear_bwd);

@@ -93,7 +93,7 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   p.staged = 0;
   const int folds = ((a->flags & kGemmResidual) != 0) + ((a->flags & kGemmGeluDual) != 0) + ((a->flags & kGemmDGelu) != 0);
   if (!(a->flags & kGemmOutF32) && folds <= 1) {      // combinations: direct stores
-    auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld % 8 == 0; };
+    auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld > 0 && ld % 8 == 0; };
     bool ok = ok16(a->C, a->ldc);
     if (a->flags & kGemmGeluDual) ok = ok && ok16(a->C2, a->ldc);
     if (a->flags & kGemmResidual) ok = ok && ok16(a->residual, a->ldr);
@@ -110,7 +110,7 @@ extern "C" int itb_gemm_bf16_pair(const ItbGemmArgs* a, cudaStream_t stream) {
   // fp32 outputs the same way, a residual of fp32 among them (not under an accumulation, where each share would add it, and
   // not where N ends off the 16 bytes that a bulk store writes whole: the columns beyond are the caller's)
   if ((a->flags & kGemmOutF32) && !(a->flags & (kGemmGeluDual | kGemmDGelu))) {
-    auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld % 4 == 0; };
+    auto ok16 = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && ld > 0 && ld % 4 == 0; };
     const bool residual = a->flags & kGemmResidual;
     if (ok16(a->C, a->ldc) && (!residual || (a->N % 4 == 0 && !(a->flags & (kGemmAtomic | kGemmAccum)) && ok16(a->residual, a->ldr)))) {
       rc = make_tmap_f32_2d(&tc, a->C, a->N, a->M, a->ldc, 32);

@@ -114,15 +114,8 @@ def _pad_cols(n: int) -> int:
 
 
 def _as_bf16_2d(x: torch.Tensor) -> torch.Tensor:
-    x2 = x.reshape(-1, x.shape[-1])
-    if x2.dtype != torch.bfloat16:
-        x2 = x2.to(torch.bfloat16)
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
-        x2 = x2.contiguous()
-    if x2.stride(0) % 8:        # TMA wants rows a multiple of 16 bytes apart; the gradient of a rank-4 product's are not
-        padded = x2.new_empty(x2.shape[0], (x2.shape[1] + 7) // 8 * 8)
-        x2 = padded[:, :x2.shape[1]].copy_(x2)
-    return x2
+    """``x`` as a bf16 matrix whose rows the kernels can read."""
+    return _C().bf16_rows(x)
 
 
 # --------------------------------------------------------------------------- linear

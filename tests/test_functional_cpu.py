@@ -273,3 +273,20 @@ def test_slot_that_a_kernel_may_add_to(how):
     elif how == "node_hook":
         accumulator.register_hook(lambda gi, go: None)
     assert C.adds_in_place(p, slot) == (how == "plain")
+
+
+def test_rows_that_a_tensor_map_can_take():
+    """Unit column stride and a pitch of whole 16 bytes, never 0; what is laid out so already is not copied."""
+    from infinitrain_b200 import _ext
+
+    C = _ext.load(required=False)
+    if C is None:
+        pytest.skip("native extension not built")
+    base = torch.randn(4, 6, 24).bfloat16()
+    for x, copied in ((base, False), (base[:, :, :8], False), (base[0, 0].expand(4, 6, 24), True), (base[0, 0].expand(5, 24), True),
+                      (base[0].t(), True), (base[..., :5], False), (base[..., 1:9], True), (base.float(), True),
+                      (torch.randn(3, 4).bfloat16(), True)):
+        y = C.bf16_rows(x)
+        assert y.dtype == torch.bfloat16 and y.stride(1) == 1 and y.stride(0) % 8 == 0 and y.stride(0) >= y.shape[1]
+        assert torch.equal(y, x.reshape(-1, x.shape[-1]).bfloat16())
+        assert (y.data_ptr() != x.data_ptr()) == copied

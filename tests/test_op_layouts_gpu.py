@@ -127,3 +127,29 @@ def test_gradient_slots_are_added_to():
     assert w.grad is None and b.grad is None and [p is q for p, q in zip(fired, (w, b))] == [True, True]
     _close(w.main_grad - 1, dw, "weight")
     _close(b.main_grad - 1, db, "bias")
+
+
+@pytest.mark.parametrize("T", [50, 800])           # 128 x 64 tiles, CTA pairs
+@pytest.mark.parametrize("residual", [None, torch.bfloat16, torch.float32])
+def test_one_row_for_all(T, residual):
+    """Gradients, inputs and residuals that are one row expanded: the rows have no pitch that a tensor map could take."""
+    torch.manual_seed(T)
+    N, K = 640, 64
+    row = lambda n, dtype: torch.randn(n, device="cuda").to(dtype).expand(3, T, n)
+    w = torch.randn(N, K, device="cuda").bfloat16().float() * 0.1
+    b = torch.randn(N, device="cuda")
+    r = row(N, residual) if residual else None
+    dys = lambda expect: {"one row": row(N, torch.bfloat16)}
+    for x in (torch.randn(3, T, K, device="cuda").bfloat16(), row(K, torch.bfloat16)):
+        _compare(lambda x, w, b, r: F.linear(x, w, b, r), lambda x, w, b, r: ref.linear(x, w, b, r, False), [x, w, b, r], dys, T)
+    _compare(lambda x, w, b: F.linear(x, w, b, gelu=True), lambda x, w, b: ref.linear(x, w, b, None, True), [x, w, b], dys, T)
+
+
+def test_sum_over_rows():
+    """The gradient of a sum over all rows of a matrix."""
+    x = torch.randn(300, 64, device="cuda").bfloat16().requires_grad_()
+    w = torch.randn(72, 64, device="cuda", requires_grad=True)
+    v = torch.randn(72, device="cuda").bfloat16()
+    (F.linear(x, w).sum(0) * v).sum().backward()
+    _close(x.grad, (v.float() @ w.detach().bfloat16().float()).expand(300, 64), "dx")
+    _close(w.grad, v.float()[:, None] * x.detach().float().sum(0), "dw")
