@@ -10,6 +10,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "ring.h"
+
 namespace itb {
 
 // Kernel attributes (the dynamic shared-memory limit) are per device: remember per device, not per
@@ -87,6 +89,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     if (i > 64) __nanosleep(32);
   }
   return false;
+}
+
+// For a launch that gives up: waits (bounded) for the loads that a producer issued into its ring and that nobody consumes any
+// more; they land in this CTA's shared memory.  After all warps are done, since any of them may be the one that gave up.
+template <int kStages>
+__device__ __forceinline__ void drain_ring(uint64_t* full_bar, uint32_t position) {
+  for (int s = 0; s < kStages; ++s) mbar_wait(&full_bar[s], ring_last_parity(s, position));
 }
 
 // ---------------------------------------------------------------- TMA

@@ -157,6 +157,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   uint64_t* operand_bar = tmem_empty + 2;         // of each epilogue warp (and slot): residual / aux tile landed
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(operand_bar + L::kOperandBars);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  volatile uint32_t* stopped_at = tmem_holder + 2;      // the TMA warp's place in the ring
 
   const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();          // 0 = leader
@@ -292,6 +293,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           }
         }
       }
+      *stopped_at = ring_position(stage, phase);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
@@ -683,6 +685,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
   tc_fence_before_sync();
   __syncthreads();
+  // (both CTAs' loads of a stage complete on the leader's barrier)
+  if (leader && threadIdx.x == 0 && *abort_flag) drain_ring<kStages>(full_bar, *stopped_at);
+  __syncwarp();
   cluster_sync_all();      // the peer may still signal this CTA's barriers until it gets here
   if (warp == 1) {
     tc_fence_after_sync();

@@ -61,6 +61,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   uint64_t* acc_full = empty_bar + kStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  volatile uint32_t* stopped_at = tmem_holder + 2;      // the TMA warp's place in the ring
 
   constexpr int kPasses = BM / 16;               // 128 threads take 16 rows of 8 x 8 columns at a time
   const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -90,12 +91,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
       for (int kb = 0; kb < p.k_blocks; ++kb) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1) || *abort_flag) {
           atomicCAS(p.err, 0, 105);
           *abort_flag = 1;
-          ok = false;
           break;
         }
         uint8_t* sa = smem + stage * kStageBytes;
@@ -117,10 +116,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           phase ^= 1;
         }
       }
-      // on the abort path: loads that were issued land in this CTA's shared memory
-      if (!ok) {
-        for (int s = 0; s < kStages; ++s) mbar_wait(&full_bar[s], phase);
-      }
+      *stopped_at = ring_position(stage, phase);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -303,6 +299,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) drain_ring<kStages>(full_bar, *stopped_at);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, BN);

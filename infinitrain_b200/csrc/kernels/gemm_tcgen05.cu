@@ -61,6 +61,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  volatile uint32_t* stopped_at = tmem_holder + 2;      // the TMA warp's place in the ring
 
   const int warp = __shfl_sync(~0u, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
@@ -148,12 +149,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
           }
         }
       }
-      // Loads still in flight land in this CTA's shared memory; the MMA warp consumes every stage
-      // that was issued before it leaves its loop, so nothing is outstanding at exit on the normal
-      // path.  On the abort path wait (bounded) for the stages that were issued.
-      if (!ok) {
-        for (int s = 0; s < kStages; ++s) mbar_wait(&full_bar[s], phase);
-      }
+      // The MMA warp consumes every stage that was issued before it leaves its loop, so nothing is outstanding at exit
+      // unless it gives up.
+      *stopped_at = ring_position(stage, phase);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -255,6 +253,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
 
   tc_fence_before_sync();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) drain_ring<kStages>(full_bar, *stopped_at);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);

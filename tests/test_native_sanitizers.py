@@ -50,6 +50,18 @@ def test_tp_protocol_model_and_its_negative_control(tmp_path):
     assert r.returncode != 0 and "protocol violations" in r.stderr
 
 
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_ring_model_and_its_negative_control(tmp_path):
+    """What a GEMM launch that gives up waits for: exactly the loads of its ring that have not landed."""
+    src = os.path.join(ROOT, "tests", "native", "ring_model.cc")
+    inc = "-I" + os.path.join(ROOT, "infinitrain_b200", "csrc", "common")
+    for flags, code in (([], 0), (["-DITB_RING_ONE_PARITY"], 1)):
+        exe = tmp_path / f"ring{code}"
+        subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", inc, *flags, src, "-o", str(exe)], check=True)
+        r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+        assert r.returncode == code and "ring model" in r.stdout, r.stdout
+
+
 @pytest.mark.skipif(shutil.which("cmake") is None, reason="needs cmake")
 def test_parallel_stack_under_thread_sanitizer(tmp_path):
     """The C++ frontend's process groups, DDP reducer, ZeRO optimizer and pipeline executor, with the
