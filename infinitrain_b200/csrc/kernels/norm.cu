@@ -464,7 +464,8 @@ partial_reduce_kernel(const float* __restrict__ partial, int prow_stride, int nr
   out[oc] = ((accumulate >> which) & 1) ? out[oc] + t : t;
 }
 
-constexpr int kWarpRowsFrom = 4096;      // rows up to 768 wide: more than this many go one to a warp
+// Rows up to 768 wide: more than this many go one to a warp (three sums of parameter gradients / fewer).
+constexpr int kBlockRowsThreeSums = 4096, kBlockRows = 448;
 
 // Upper bound of the backward grid for `rows` rows in either layout: what callers size `partial` with.
 static int norm_grid(int rows) { return rows < kMaxPartialRows ? (rows < 1 ? 1 : rows) : kMaxPartialRows; }
@@ -524,10 +525,17 @@ static int norm_bwd_dispatch(const void* dy, int dyd, const void* x, int xd, con
   if (C % 8 || C > 6144) return -3;
   if (rows < 1) return 0;
   // One warp per row keeps a row's sums inside the warp, but pays at the end for warps that add their parameter gradients up
-  // in turns, and 128 columns a warp past 768 take a fourth chunk and its registers.  us with a warp / a block per row,
-  // bf16 with a residual's gradient: 96 x 768 21.4 / 13.0, 2331 x 768 23.6 / 21.6, 4096 x 768 25.6 / 25.5, 8192 x 768 31.7 / 31.7,
-  // 16384 x 768 42.1 / 46.0, 8192 x 1024 58.3 / 35.8.
-  const bool wide = C > 768 || rows <= kWarpRowsFrom;
+  // in turns, gamma's, beta's and the residual's one after the other; a block per row pays two barriers a row and up to
+  // twice the partial rows.  So a block for each of few rows, of more only where there are three sums; and 128 columns a
+  // warp past 768 take a fourth chunk and its registers.  us with a warp / a block per row, reduction of the parameter
+  // gradients included, one launch after another on bf16:
+  //   three sums     96 x 768 14.0 / 6.2, 512 x 128 7.1 / 6.7, 1536 x 256 9.5 / 9.2, 4096 x 384 14.5 / 13.7, 4096 x 768 19.2 / 17.8;
+  //                  with 8192 rows of 256 columns the warp is ahead (13.7 / 14.5), from L2's size on at 768 too (16384 x 768 42.1 / 46.0)
+  //   layer norm     384 x 128 7.0 / 5.5, 384 x 768 12.4 / 9.9, 512 x 128 6.3 / 7.1, 512 x 768 12.1 / 13.1, 4096 x 256 9.8 / 11.6
+  //   RMS, residual  384 x 128 6.6 / 5.5, 384 x 768 12.4 / 10.0, 512 x 256 7.0 / 8.0, 1536 x 512 11.5 / 12.2, 4096 x 768 16.2 / 16.9
+  //   RMS            384 x 128 6.1 / 5.5, 384 x 768 10.2 / 9.6, 512 x 768 9.8 / 12.7, 4096 x 768 13.7 / 16.7
+  // and 8192 x 1024 58.3 / 35.8.
+  const bool wide = C > 768 || rows <= (!kRms && dres ? kBlockRowsThreeSums : kBlockRows);
   int grid = 0;
 #define LAUNCH_K(TDY, TX, TDX, CH, RES, WIDE)                                                     \
   do {                                                                                            \

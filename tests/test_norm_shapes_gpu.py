@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(1, 8), (3, 768), (4096, 768), (4097, 768), (5000, 264), (700, 776), (600, 1024), (301, 1032), (1500, 2048), (900, 2056),
+SIZES = [(1, 8), (3, 768), (448, 512), (449, 512), (449, 768), (4096, 768), (4097, 768), (5000, 264), (700, 776), (600, 1024), (301, 1032), (1500, 2048), (900, 2056),
          (700, 4096), (300, 4104), (250, 6144)]
 
 
