@@ -11,7 +11,6 @@ bf16 between the fused kernels.
 from __future__ import annotations
 
 import functools
-import math
 from typing import Optional
 
 import torch
@@ -72,11 +71,6 @@ def _apply(fn, *args):
             or torch._C._get_tracing_state() is not None or torch._C._autograd._profiler_enabled()):
         return fn.apply(*args)
     return fn.forward(_NoContext(), *args)
-
-
-def _heads(qkv: torch.Tensor, H: int, KV: int, D: int):
-    """Query, key and value heads ``[B, T, heads, D]`` of a packed projection, as views."""
-    return qkv.view(*qkv.shape[:-1], H + 2 * KV, D).split((H, KV, KV), dim=-2)
 
 
 # --------------------------------------------------------------------------- bf16 weight shadows
@@ -246,16 +240,10 @@ def _grad_written(p: torch.Tensor) -> None:
         hook(p)
 
 
-def _bias_grad(C, dy2, N, bias=None):
-    """Column sums of dY.  With a flat gradient buffer behind ``bias`` they are added straight into
-    its slot (no gradient tensor, no separate accumulation launch) and None is returned."""
+def _bias_grad(C, dy2, N):
+    """Column sums of dY."""
     if N % 8 == 0 and dy2.data_ptr() % 16 == 0:
         _counters["launches"] += 2
-        main = _main_grad_of(bias)
-        if main is not None:
-            C.colsum(dy2, main)
-            _grad_written(bias)
-            return None
         return C.colsum(dy2)
     return dy2.float().sum(0)
 
