@@ -685,13 +685,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
   tc_fence_before_sync();
   __syncthreads();
-  // (both CTAs' loads of a stage complete on the leader's barrier)
-  if (leader && threadIdx.x == 0 && *abort_flag) drain_ring<kStages>(full_bar, *stopped_at);
-  __syncwarp();
   cluster_sync_all();      // the peer may still signal this CTA's barriers until it gets here
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem_base, kTmemCols);
+  }
+  // Beside the other warp's deallocation, where it costs a launch that succeeds nothing (ahead of the cluster's barrier: 0.08 us).
+  // Both CTAs' loads of a stage complete on the leader's barrier; the other CTA gives its own a millisecond.
+  if (threadIdx.x == 0 && *abort_flag) {
+    if (leader) {
+      drain_ring<kStages>(full_bar, *stopped_at);
+    } else {
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
   }
   if constexpr (kTp) {
     if (tp.mode & kTpScatter) {
