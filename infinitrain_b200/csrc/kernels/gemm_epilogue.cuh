@@ -63,7 +63,7 @@ __device__ __forceinline__ float dgelu_tanh(float x) {
   const float x2 = x * x;
   const float t = tanh_fast(x * fmaf(x2, k0 * k1, k0));
   // 0.5 x u' meets 1 - t^2 one factor at a time: whole it is infinite from 2e13 on, where 1 - t^2 is zero
-  return fmaf(fmaf(-t, t, 1.f) * x, fmaf(x2, 1.5f * k0 * k1, 0.5f * k0), fmaf(0.5f, t, 0.5f));
+  return fmaf(fmaf(-t, t, 1.f) * fmaf(x2, 1.5f * k0 * k1, 0.5f * k0), x, fmaf(0.5f, t, 0.5f));
 }
 
 // v: 32 consecutive accumulator columns [col0, col0 + 32) of output row `row`.
