@@ -668,7 +668,7 @@ std::tuple<OptTensor, OptTensor, OptTensor> linear_bwd(const at::Tensor& dy, con
   OptTensor dx, dw, db;
   if (w) {
     dx = at::empty(sizes_with_last(dy, K), dy2.options());
-    Gemm(dy2, false, *w, true, M, K, N).into(dx->data_ptr(), K).run();
+    Gemm(dy2, false, *w, true, M, K, N).into(dx->data_ptr(), K, kGemmMaySplit).run();
   }
   if (want_dw) dw = weight_grad(dy2, x2, main_dw, dw_ready);
   if (want_db) db = bias_grad(dy2, main_db, db_ready);
@@ -707,7 +707,7 @@ std::tuple<OptTensor, OptTensor, OptTensor, OptTensor, OptTensor> mlp_gelu_bwd(
   const int64_t M = x2.size(0), C = x2.size(1), F = h.size(1);
   at::Tensor dh = at::empty({M, F}, dy2.options());
   Gemm g(dy2, false, w_proj, true, M, F, C);      // the derivative is applied in the epilogue
-  g.into(dh.data_ptr(), F, kGemmDGelu);
+  g.into(dh.data_ptr(), F, kGemmDGelu | kGemmMaySplit);
   g.aux = h.data_ptr();
   g.ld_aux = h.stride(0);
   g.run();
@@ -716,7 +716,7 @@ std::tuple<OptTensor, OptTensor, OptTensor, OptTensor, OptTensor> mlp_gelu_bwd(
   if (want_db_proj) db_proj = bias_grad(dy2, main_b_proj, b_proj_ready);
   if (want_dx) {
     dx = at::empty(sizes_with_last(dy, C), dy2.options());
-    Gemm(dh, false, w_fc, true, M, C, F).into(dx->data_ptr(), C).run();
+    Gemm(dh, false, w_fc, true, M, C, F).into(dx->data_ptr(), C, kGemmMaySplit).run();
   }
   if (want_dw_fc) dw_fc = weight_grad(dh, x2, main_fc, fc_ready);
   if (want_db_fc) db_fc = bias_grad(dh, main_b_fc, b_fc_ready);
@@ -767,6 +767,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("GEMM_OUT_F32") = static_cast<int>(kGemmOutF32);
   m.attr("GEMM_ATOMIC") = static_cast<int>(kGemmAtomic);
   m.attr("GEMM_FRESH") = static_cast<int>(kGemmFresh);
+  m.attr("GEMM_MAY_SPLIT") = static_cast<int>(kGemmMaySplit);
   m.attr("GEMM_ACCUM") = static_cast<int>(kGemmAccum);
   m.attr("GEMM_BIAS") = static_cast<int>(kGemmBias);
   m.attr("GEMM_RESIDUAL") = static_cast<int>(kGemmResidual);

@@ -184,7 +184,7 @@ struct LinearFn : public torch::autograd::Function<LinearFn> {
     if (ctx->needs_input_grad(0)) {
       Tensor w = weight_lp(weight);
       Tensor dx2 = torch::empty({M, K}, dy2.options());
-      gemm(dy2, false, w, true, M, K, N, dx2, Tensor(), Tensor(), Tensor(), Tensor(), 0);
+      gemm(dy2, false, w, true, M, K, N, dx2, Tensor(), Tensor(), Tensor(), Tensor(), kGemmMaySplit);
       dx = dx2.view(ctx->saved_data["x_shape"].toIntVector());
       if (!ctx->saved_data["x_bf16"].toBool()) dx = dx.to(torch::kFloat32);
     }

@@ -22,6 +22,7 @@ enum {
   kGemmGeluDual = 32,  // C = h (bf16), C2 = gelu_tanh(h) (bf16)
   kGemmDGelu = 64,     // C = (A*B) * gelu_tanh'(aux[m,n])
   kGemmFresh = 128,    // with kGemmAtomic: C holds nothing yet; cleared where the contraction is split, else stored to
+  kGemmMaySplit = 256, // a small output's contraction may be split (gradients): a row's last bits then depend on M
   // Timing probes of the CTA-pair pipeline (results are meaningless): the same launch with the
   // operand loads left out (the MMA warp finds every stage "full" at once: issue rate + shared-memory
   // reads of the tensor core alone) or with the MMAs left out (TMA fill rate of the ring alone).
@@ -53,7 +54,8 @@ typedef struct {
 int itb_gemm_bf16(const ItbGemmArgs* args, cudaStream_t stream);
 // Whether the output is small enough for 128 x 64 tiles to run all at once (and nothing is accumulated) ...
 int itb_gemm_is_small(const ItbGemmArgs* args);
-// ... and the kernel for it (gemm_small.cu), to which the other two entries hand such outputs.  split_k is not looked at.
+// ... and the kernel for it (gemm_small.cu), to which the other two entries hand such outputs.  split_k, with kGemmMaySplit:
+// into how many shares (1, 2, 4, 8) the contraction is dealt out, 0 = choose.
 int itb_gemm_small(const ItbGemmArgs* args, cudaStream_t stream);
 // Same contract, computed by CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles per pair) unless the output is that small.
 // Where C (and C2) are on 16 bytes with rows a multiple of 16 bytes apart, a row's last bulk store writes its 16 bytes whole:

@@ -33,3 +33,27 @@ def test_rows_do_not_depend_on_their_number(N, K, kind):
             want = torch.cat((whole[:rows], whole[most:most + rows])) if kind == "gelu" else whole[:rows]
             assert torch.equal(got, want), rows
     assert C.kernel_status() == 0
+
+
+def test_only_gradients_are_split():
+    """Splitting is the caller's to allow, whatever number of shares is asked for; a linear's input gradient allows it."""
+    from infinitrain_b200 import _ext
+    from infinitrain_b200.ops import functional as F
+
+    C = _ext.load(required=True)
+    torch.manual_seed(5)
+    x = torch.randn(96, 3072, device="cuda").bfloat16()
+    w = torch.randn(768, 3072, device="cuda").bfloat16()
+
+    def product(flags, shares):
+        out = torch.empty(96, 768, device="cuda", dtype=torch.bfloat16)
+        C.gemm(x, False, w, False, 96, 768, 3072, out, None, None, None, None, flags, shares)
+        return out
+
+    whole, split = product(0, 0), product(C.GEMM_MAY_SPLIT, 0)
+    assert torch.equal(product(0, 8), whole) and torch.equal(product(C.GEMM_MAY_SPLIT, 1), whole)
+    assert torch.equal(product(C.GEMM_MAY_SPLIT, 8), split) and not torch.equal(split, whole)
+    assert torch.equal(F.linear(x, w), whole)
+    z = torch.zeros(96, 768, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    F.linear(z, w.t().contiguous()).backward(x)         # the same product as an input gradient
+    assert torch.equal(z.grad, split)

@@ -1,24 +1,25 @@
-"""The GEMM for outputs of at most one wave of 128 x 64 tiles: every order of the operands with every epilogue, at sizes with
-remainders, against 64 bits."""
+"""The GEMM for outputs of at most one wave of 128 x 64 tiles: every order of the operands and every number of shares of the
+contraction with every epilogue, at sizes with remainders, against 64 bits."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# (M, N, K): one row; ragged tiles and k-blocks; a few k-blocks, fewer than the ring has stages
+# (M, N, K): one row; ragged tiles and shares of unequal length; shares of one k-block; a row of clusters
 SIZES = [(1, 8, 1544), (130, 72, 520), (257, 200, 1096), (96, 768, 512), (300, 1001, 640)]
 KINDS = ["plain", "bias", "bias32", "residual", "residual32", "gelu", "dgelu", "unaligned", "unaligned32", "gelu_residual"]
 
 
+@pytest.mark.parametrize("shares", [0, 1, 2, 4, 8])
 @pytest.mark.parametrize("b_mn", [False, True], ids=["b_k_major", "b_mn_major"])
 @pytest.mark.parametrize("a_mn", [False, True], ids=["a_k_major", "a_mn_major"])
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("M,N,K", SIZES)
-def test_small_gemm(M, N, K, kind, a_mn, b_mn):
+def test_small_gemm(M, N, K, kind, a_mn, b_mn, shares):
     from infinitrain_b200 import _ext
 
     C = _ext.load(required=True)
-    torch.manual_seed(M + N)
+    torch.manual_seed(M + N + shares)
     ld = (N + 63) // 64 * 64 + (1 if "unaligned" in kind else 0)       # odd rows: element by element
     dtype = torch.float32 if "32" in kind else torch.bfloat16
     a = torch.randn(K, (M + 7) // 8 * 8, device="cuda").bfloat16()[:, :M]         # rows a multiple of 16 bytes apart
@@ -26,7 +27,7 @@ def test_small_gemm(M, N, K, kind, a_mn, b_mn):
     bias = torch.randn(N, device="cuda")
     operand = torch.randn(M, ld, device="cuda").to(dtype)[:, :N]
     exact = a.double().t() @ b.double()
-    flags = C.GEMM_OUT_F32 if dtype == torch.float32 else 0
+    flags = (C.GEMM_OUT_F32 if dtype == torch.float32 else 0) | (C.GEMM_MAY_SPLIT if shares else 0)
     if kind not in ("plain", "dgelu"):
         flags |= C.GEMM_BIAS
         exact = exact + bias.double()
@@ -40,12 +41,12 @@ def test_small_gemm(M, N, K, kind, a_mn, b_mn):
         out, out2 = (torch.full((M, ld), float("nan"), device="cuda", dtype=dtype) for _ in range(2))
         C.gemm(a if a_mn else a.t().contiguous(), a_mn, b if b_mn else b.t().contiguous(), b_mn, M, N, K, out,
                out2 if flags & C.GEMM_GELU_DUAL else None, bias, operand if flags & C.GEMM_RESIDUAL else None,
-               operand if kind == "dgelu" else None, flags, 0)
+               operand if kind == "dgelu" else None, flags, shares)
         outs.append((out, out2))
     torch.cuda.synchronize()
     assert C.kernel_status() == 0
     out, out2 = outs[0]
-    assert torch.equal(out[:, :N], outs[1][0][:, :N])          # the same bits every time
+    assert torch.equal(out[:, :N], outs[1][0][:, :N])          # the shares are added in one order
     assert torch.isnan(out[:, N:].float()).all()
 
     got = out[:, :N].double()
